@@ -77,6 +77,36 @@ template <bool kSelect = true>
 __device__ __forceinline__ uint64_t mass_of(float x) {
     return __float2ull_rn(__fmul_rn(exp_det<kSelect>(x), 1099511627776.0f));
 }
+// The masses of two tokens at once, from their logits: (z - m) * inv_T, exp_det and the scaling by
+// 2^40 as packed fp32x2 operations -- every lane of a packed operation rounds like the scalar one,
+// so the bits are those of mass_of(scaled_shift(z, m, inv_T)).  The whole-distribution kernels are
+// bound by issue slots (27 instructions per token in scalar form); packed they take 13.  No test
+// of the range: an argument below -80, or NaN, is clamped to -80, whose mass rounds to 0 as well.
+__device__ __forceinline__ float2 exp_det2(float2 x) {
+    x.x = fmaxf(x.x, -80.0f);
+    x.y = fmaxf(x.y, -80.0f);
+    const float magic = 12582912.0f;
+    const float2 r = __fadd2_rn(__fmul2_rn(x, make_float2(0x1.715476p+0f, 0x1.715476p+0f)), make_float2(magic, magic));
+    const float2 nf = __fadd2_rn(r, make_float2(-magic, -magic));
+    float2 f = __ffma2_rn(nf, make_float2(-0x1.62e4p-1f, -0x1.62e4p-1f), x);
+    f = __ffma2_rn(nf, make_float2(-0x1.7f7d1cp-20f, -0x1.7f7d1cp-20f), f);
+    float2 p = make_float2(0x1.687bf6p-10f, 0x1.687bf6p-10f);
+    p = __ffma2_rn(p, f, make_float2(0x1.123b9ep-7f, 0x1.123b9ep-7f));
+    p = __ffma2_rn(p, f, make_float2(0x1.555b58p-5f, 0x1.555b58p-5f));
+    p = __ffma2_rn(p, f, make_float2(0x1.55548ep-3f, 0x1.55548ep-3f));
+    p = __ffma2_rn(p, f, make_float2(0x1.fffff8p-2f, 0x1.fffff8p-2f));
+    p = __ffma2_rn(p, f, make_float2(1.0f, 1.0f));
+    p = __ffma2_rn(p, f, make_float2(1.0f, 1.0f));
+    // (n << 23 with n = bits(r) - 0x4B400000: the constant shifts out)
+    return make_float2(__uint_as_float(__float_as_uint(p.x) + (__float_as_uint(r.x) << 23)),
+                       __uint_as_float(__float_as_uint(p.y) + (__float_as_uint(r.y) << 23)));
+}
+__device__ __forceinline__ void mass2_of(float2 z, float m, float inv_T, uint64_t& q0, uint64_t& q1) {
+    const float2 x = __fmul2_rn(__fadd2_rn(z, make_float2(-m, -m)), make_float2(inv_T, inv_T));
+    const float2 e = __fmul2_rn(exp_det2(x), make_float2(1099511627776.0f, 1099511627776.0f));
+    q0 = __float2ull_rn(e.x);
+    q1 = __float2ull_rn(e.y);
+}
 // x = (z - m) * inv_T with two roundings
 __device__ __forceinline__ float scaled_shift(float z, float m, float inv_T) {
     return __fmul_rn(__fsub_rn(z, m), inv_T);
