@@ -96,7 +96,9 @@ __device__ __forceinline__ void draw_weight2(const DrawCtx& D, float2 zp, float2
 // The blocks of all rows form one sequence, dealt to all warps of the grid in contiguous, equal
 // ranges; a warp streams its blocks through its own ring (warp_ring.cuh) and never meets another
 // warp.  Bound by the fp32 pipe and issue slots of the deterministic exp (13 instructions per token
-// in packed form), then by HBM: one pass, every logit read once.
+// in packed form, 27 before), then by HBM: one pass, every logit read once.  32 sequences of five
+// draft tokens over 128256-token rows (180.6 MB): 90.6 us before, 53.0 us now, both launches; tiles
+// of 8192 tokens behind a block-wide barrier each had left the pipes idle while the warps met.
 struct MassShared {
     unsigned long long bars[kSpecStages * (kSpecThreads / 32)];
 };
