@@ -46,10 +46,10 @@ struct Handle {
     int num_sms = 0;
     int max_grid = 0;              // CTAs of the streaming kernel (two per SM)
     int max_rows = 0;              // virtual rows (caller rows x vocabulary segments) a call may stream
-    int rec_cap = 0;               // entries per segment record
-    int64_t rec_stride = 0;
-    size_t records_bytes = 0;
-    uint8_t* records = nullptr;    // segment records, indexed by row + cta
+    int rec_slots = 0;             // segment records there is room for
+    uint8_t* records = nullptr;    // segment records (kSegRecordBytes each)
+    uint16_t* gkeys = nullptr;     // group keys of rows that several CTAs stream
+    int64_t gkeys_cap = 0;
     MassBlock* blocks = nullptr;   // mass blocks of the whole-vocabulary routes
     int64_t blocks_cap = 0;
     uint32_t* tickets = nullptr;   // [max_rows] tickets, then [max_rows] deferred-fallback owners
@@ -174,52 +174,33 @@ bool host_need_mass(const born_row_params& p) {
 // The dynamic shared-memory limit of every instantiation is raised once (at create / first static call).
 cudaError_t scan_attrs_all() {
     cudaError_t e;
-    if ((e = scan_attrs_f32_pair()) != cudaSuccess) return e;
-    if ((e = scan_attrs_f32_pair_row()) != cudaSuccess) return e;
+    if ((e = scan_attrs_f32()) != cudaSuccess) return e;
     if ((e = scan_attrs_f32_hist()) != cudaSuccess) return e;
-    if ((e = scan_attrs_f32_hist_row()) != cudaSuccess) return e;
-    if ((e = scan_attrs_f32_hist_short_row()) != cudaSuccess) return e;
-    if ((e = scan_attrs_bf16_pair()) != cudaSuccess) return e;
-    if ((e = scan_attrs_bf16_pair_row()) != cudaSuccess) return e;
+    if ((e = scan_attrs_f32_mask()) != cudaSuccess) return e;
+    if ((e = scan_attrs_f32_mask_hist()) != cudaSuccess) return e;
     if ((e = scan_attrs_bf16()) != cudaSuccess) return e;
-    return scan_attrs_bf16_row();
+    if ((e = scan_attrs_bf16_hist()) != cudaSuccess) return e;
+    if ((e = scan_attrs_bf16_mask()) != cudaSuccess) return e;
+    return scan_attrs_bf16_mask_hist();
 }
 
 // The route class of a launch (RouteOf in scan_common.cuh): uniform parameters tell it on the host.
 static int route_of(const born_row_params* row_params, const born_row_params& p) {
     if (row_params) return 0;
-    if (host_need_mass(p)) return 0;
-    const bool greedy = (p.flags & BORN_FLAG_GREEDY) || p.temperature == 0.0f;
-    return (!greedy && p.top_k > 0) ? 2 : 1;
+    return host_need_mass(p) ? 2 : 1;
 }
 
-int launch_scan(Handle* h, const ScanArgs& A, int dtype, int grid, cudaStream_t st) {
+int launch_scan(Handle* h, const ScanArgs& A, int dtype, bool aligned, int grid, cudaStream_t st) {
     const int route = route_of(A.row_params, A.params);
-    const bool has_mask = A.mask != nullptr;
-    const bool lse = A.out_lse != nullptr || A.want_lse;
-
-    // Launches without a token history take the instantiations that carry no history code (fp32:
-    // their loop pairs tiles); launches with one take the others.
-    // A sampling launch whose grid is one CTA per row (the tile ranges of range_begin are then the
-    // rows themselves) takes the instantiations without the segment-record path.
-    const bool one_row = A.mode == kScanFull && A.G == 1 && grid == A.B;
-    // ... and, fp32 with histories of at most kHistShort ids per row, the one whose list takes half the room
-    const bool short_hist = one_row && dtype == BORN_DTYPE_F32 && A.history != nullptr && A.history_stride <= kHistShort;
-    const size_t smem = (size_t)scan_smem_layout(dtype == BORN_DTYPE_F32 ? 4 : 2, has_mask, A.history != nullptr,
-                                                 short_hist ? kHistShort : (int)BORN_MAX_HISTORY).total;
+    const bool mask = A.mask != nullptr, hist = A.history != nullptr;
     cudaError_t e;
-    if (dtype != BORN_DTYPE_F32 && A.history == nullptr)
-        e = one_row ? scan_launch_bf16_pair_row(A, has_mask, lse, route, grid, smem, st)
-                    : scan_launch_bf16_pair(A, has_mask, lse, route, grid, smem, st);
-    else if (dtype != BORN_DTYPE_F32)
-        e = one_row ? scan_launch_bf16_row(A, has_mask, lse, route, grid, smem, st) : scan_launch_bf16(A, has_mask, lse, route, grid, smem, st);
-    else if (A.history == nullptr)
-        e = one_row ? scan_launch_f32_pair_row(A, has_mask, lse, route, grid, smem, st)
-                    : scan_launch_f32_pair(A, has_mask, lse, route, grid, smem, st);
-    else
-        e = short_hist ? scan_launch_f32_hist_short_row(A, has_mask, lse, route, grid, smem, st)
-            : one_row  ? scan_launch_f32_hist_row(A, has_mask, lse, route, grid, smem, st)
-                       : scan_launch_f32_hist(A, has_mask, lse, route, grid, smem, st);
+    if (dtype == BORN_DTYPE_F32) {
+        if (mask) e = hist ? scan_launch_f32_mask_hist(A, aligned, route, grid, st) : scan_launch_f32_mask(A, aligned, route, grid, st);
+        else e = hist ? scan_launch_f32_hist(A, aligned, route, grid, st) : scan_launch_f32(A, aligned, route, grid, st);
+    } else {
+        if (mask) e = hist ? scan_launch_bf16_mask_hist(A, aligned, route, grid, st) : scan_launch_bf16_mask(A, aligned, route, grid, st);
+        else e = hist ? scan_launch_bf16_hist(A, aligned, route, grid, st) : scan_launch_bf16(A, aligned, route, grid, st);
+    }
     if (e != cudaSuccess) return fail(h, BORN_ERR_CUDA, "scan kernel launch failed: %s", cudaGetErrorString(e));
     h->launches++;
     return BORN_OK;
@@ -232,42 +213,54 @@ int launch_merge(Handle* h, const MergeArgs& M, cudaStream_t st) {
     return BORN_OK;
 }
 
+// Whether every virtual row starts on a 16-byte boundary.
+bool rows_aligned(int G, int V, int dtype, const void* logits, int64_t row_stride) {
+    const int esz = dtype == BORN_DTYPE_F32 ? 4 : 2;
+    return ((uintptr_t)logits % 16 == 0) && ((row_stride * esz) % 16 == 0) && (G == 1 || ((int64_t)V * esz) % 16 == 0);
+}
+
+// Blocks a CTA is given at least when a row is cut into slices: two per warp.  Below that a CTA
+// more saves less streaming time than the exchange through scratch costs.
+constexpr int kMinSliceBlocks = 16;
+
 // Geometry and scratch of one streaming launch over B x G virtual rows of V tokens.
 int fill_scan(Handle* h, ScanArgs& A, int B, int G, int V, int dtype, const void* logits, int64_t row_stride,
-              const uint32_t* mask, int64_t mask_stride, int* grid) {
+              const uint32_t* mask, int64_t mask_stride, int hist_cap, int* grid) {
     const int esz = dtype == BORN_DTYPE_F32 ? 4 : 2;
     if ((uintptr_t)logits % esz) return fail(h, BORN_ERR_INVALID_ARGUMENT, "logits pointer is not aligned to its element size");
     if (mask && (uintptr_t)mask % 4) return fail(h, BORN_ERR_INVALID_ARGUMENT, "mask pointer is not 4-byte aligned");
-    bool fast = ((uintptr_t)logits % 16 == 0) && ((row_stride * esz) % 16 == 0) && (G == 1 || ((int64_t)V * esz) % 16 == 0);
-    if (mask) fast = fast && ((uintptr_t)mask % 16 == 0) && ((mask_stride * 4) % 16 == 0) && (G == 1 || V % 128 == 0);
-    const int tile = kTileBytes / esz;
-    const int lead_max = fast ? 0 : 16 / esz - 1;
     A.B = B; A.G = G; A.V = V;
-    A.tpr = (int)(((int64_t)V + lead_max + tile - 1) / tile);
-    A.fast = fast ? 1 : 0;
+    A.nb = (V + kBlkTok - 1) / kBlkTok;
     A.logits = logits; A.row_stride = row_stride;
     A.mask = mask; A.mask_stride = mask_stride;
     const int64_t rows = (int64_t)B * G;
     if (rows > h->max_rows) return fail(h, BORN_ERR_UNSUPPORTED, "%lld rows (batch x segments) exceed the workspace of %d", (long long)rows, h->max_rows);
     A.nblk = (V + kMassBlock - 1) / kMassBlock;
     if (rows * A.nblk > h->blocks_cap) return fail(h, BORN_ERR_UNSUPPORTED, "batch x vocab exceeds the workspace");
-    const int64_t tiles = rows * A.tpr;
-    *grid = (int)(tiles < h->max_grid ? tiles : h->max_grid);
-    // When a whole number S of equal slices per row nearly fills the GPU, every CTA gets exactly
-    // one slice: no CTA meets a row boundary in mid-stream, and with S = 1 a row is finished from
-    // the shared memory of the CTA that streamed it.
-    for (int S = 1; S <= 64 && rows * S <= h->max_grid; ++S)
-        if (A.tpr % S == 0 && rows * S * 20 >= (int64_t)h->max_grid * 17) { *grid = (int)(rows * S); break; }
-    // entries per segment record: as many as the record area gives every (row + cta) slot
-    int64_t cap = ((int64_t)(h->records_bytes / (size_t)(rows + *grid)) - kRecordHdrBytes) / 8;
-    cap = (cap < h->rec_cap ? cap : h->rec_cap) & ~(int64_t)1;
-    if (cap < 64) return fail(h, BORN_ERR_UNSUPPORTED, "%lld rows (batch x segments) exceed the record workspace", (long long)rows);
-    A.records = h->records; A.rec_cap = (int)cap; A.rec_stride = kRecordHdrBytes + cap * 8;
+    if (rows <= h->max_grid) {
+        // every row gets CTAs of its own, as many equal slices as the GPU holds at once
+        int64_t s = h->max_grid / rows;
+        const int64_t most = (A.nb + kMinSliceBlocks - 1) / kMinSliceBlocks;
+        if (s > most) s = most;
+        if (s > 1 && rows * s > h->rec_slots) s = h->rec_slots / rows;
+        A.slices = s > 1 ? (int)s : 1;
+        *grid = (int)rows * A.slices;
+    } else {
+        A.slices = 0;
+        *grid = h->max_grid;
+    }
+    A.L = scan_smem_layout(esz, rows_aligned(G, V, dtype, logits, row_stride), mask != nullptr, hist_cap, A.slices > 0, A.slices > 1 ? 0 : A.nb * 32,
+                           kScanSmemTwo);
+    if (A.L.total > kScanSmemMax) return fail(h, BORN_ERR_UNSUPPORTED, "shared memory layout of %d bytes", A.L.total);
+    if ((A.slices != 1 || A.nb * 32 > A.L.gkeys_cap) && rows * A.nb * 32 > h->gkeys_cap)
+        return fail(h, BORN_ERR_UNSUPPORTED, "batch x vocab exceeds the workspace");
+    A.records = h->records;
+    A.gkeys = h->gkeys;
     A.blocks = h->blocks;
     A.tickets = h->tickets; A.deferred = h->tickets + h->max_rows;
     A.dev_error = h->dev_error;
     A.timeout_ns = h->timeout_ns;
-    A.debug_skip_tile = -1;
+    A.debug_skip_blk = -1;
     return BORN_OK;
 }
 
@@ -294,24 +287,24 @@ __global__ void debug_mass_kernel(const float* x, unsigned long long* q, int64_t
 
 // scratch sizes of a handle for max_batch rows of max_vocab tokens
 struct ScratchPlan {
-    int max_rows, rec_cap;
-    int64_t rec_stride, blocks_cap;
-    size_t records, blocks, tickets, seg_packed, hist, total;
+    int max_rows, rec_slots;
+    int64_t blocks_cap, gkeys_cap;
+    size_t records, gkeys, blocks, tickets, seg_packed;
 };
-ScratchPlan scratch_plan(int max_batch, int max_vocab, int max_grid, int rec_cap) {
+ScratchPlan scratch_plan(int max_batch, int max_vocab, int max_grid) {
     ScratchPlan p;
-    // virtual rows (caller rows x vocabulary segments); the record area is sized for full-size
-    // records of 2 * max_batch rows and is cut finer when a call streams more rows than that
+    // virtual rows (caller rows x vocabulary segments)
     p.max_rows = max_batch * BORN_MAX_SHARDS > 1024 ? max_batch * BORN_MAX_SHARDS : 1024;
-    p.rec_cap = rec_cap;
-    p.rec_stride = kRecordHdrBytes + (int64_t)rec_cap * 8;
-    p.records = (size_t)((max_batch * 2 > 1024 ? max_batch * 2 : 1024) + max_grid) * (size_t)p.rec_stride;
+    p.rec_slots = 2 * max_grid;  // (a CTA holds at most two rows in part)
+    p.records = (size_t)p.rec_slots * (size_t)kSegRecordBytes;
     // a call of B x G rows of V tokens needs B*G*ceil(V/512) blocks; segments only shorten V
     p.blocks_cap = (int64_t)max_batch * (((int64_t)max_vocab + kMassBlock - 1) / kMassBlock) + p.max_rows;
     p.blocks = (size_t)p.blocks_cap * sizeof(MassBlock);
+    // ... and B*G*ceil(V/1024) blocks of 32 group keys
+    p.gkeys_cap = (p.blocks_cap / 2 + p.max_rows) * 32;
+    p.gkeys = (size_t)p.gkeys_cap * sizeof(uint16_t);
     p.tickets = sizeof(uint32_t) * 2 * (size_t)p.max_rows;
     p.seg_packed = (size_t)max_batch * (size_t)(kRecordHdrBytes * BORN_MAX_SHARDS + 8 * BORN_MAX_CANDIDATES);
-    p.total = p.records + p.blocks + p.tickets + p.seg_packed + 256;
     return p;
 }
 
@@ -350,14 +343,14 @@ int32_t born_sampler_create(int32_t device, int32_t max_batch, int32_t max_vocab
     h->num_sms = prop.multiProcessorCount;
     h->max_grid = 2 * h->num_sms;
     if (cudaSetDevice(device) != cudaSuccess) { delete h; return fail(nullptr, BORN_ERR_CUDA, "cudaSetDevice failed"); }
-    const ScratchPlan sp = scratch_plan(max_batch, max_vocab, h->max_grid, 2048);
+    const ScratchPlan sp = scratch_plan(max_batch, max_vocab, h->max_grid);
     h->max_rows = sp.max_rows;
-    h->rec_cap = sp.rec_cap;
-    h->rec_stride = sp.rec_stride;
-    h->records_bytes = sp.records;
+    h->rec_slots = sp.rec_slots;
+    h->gkeys_cap = sp.gkeys_cap;
     h->blocks_cap = sp.blocks_cap;
     h->seg_packed_bytes = sp.seg_packed;
     int rc = dev_alloc(h, (void**)&h->records, sp.records);
+    if (rc == BORN_OK) rc = dev_alloc(h, (void**)&h->gkeys, sp.gkeys);
     if (rc == BORN_OK) rc = dev_alloc(h, (void**)&h->blocks, sp.blocks);
     if (rc == BORN_OK) rc = dev_alloc(h, (void**)&h->tickets, sp.tickets);
     if (rc == BORN_OK) rc = dev_alloc(h, (void**)&h->seg_packed, sp.seg_packed);
@@ -390,6 +383,7 @@ int32_t born_sampler_destroy(void* handle) {
     if (h->mask_stream) cudaStreamDestroy(h->mask_stream);
     if (h->mask_event) cudaEventDestroy(h->mask_event);
     cudaFree(h->records);
+    cudaFree(h->gkeys);
     cudaFree(h->blocks);
     cudaFree(h->tickets);
     cudaFree(h->seg_packed);
@@ -454,10 +448,11 @@ static int sample_device(Handle* h, const born_sample_args* a_in, cudaStream_t s
     memset(&A, 0, sizeof A);
     int grid = 0;
     const int G = a->vocab_segments > 1 ? a->vocab_segments : 1;
+    bool aligned = rows_aligned(G, a->vocab / G, a->logits_dtype, a->logits, a->logits_row_stride);
     int rc = fill_scan(h, A, a->batch, G, a->vocab / G, a->logits_dtype, a->logits, a->logits_row_stride, a->mask,
-                       a->mask_row_stride, &grid);
+                       a->mask_row_stride, a->history ? a->history_stride : 0, &grid);
     if (rc) return rc;
-    if (wants_clean_copy(a, A.fast != 0)) {
+    if (wants_clean_copy(a, aligned)) {
         const int64_t v_pad = ((int64_t)a->vocab + 3) / 4 * 4;
         const size_t need = (size_t)a->batch * (size_t)v_pad * sizeof(float);
         if ((rc = grow(h, (void**)&h->clean_copy, &h->clean_copy_bytes, need, st))) return rc;
@@ -479,7 +474,8 @@ static int sample_device(Handle* h, const born_sample_args* a_in, cudaStream_t s
         a2.mask = nullptr; a2.mask_row_stride = 0;
         a2.history = nullptr; a2.history_len = nullptr; a2.history_stride = 0;
         a = &a2;
-        rc = fill_scan(h, A, a->batch, 1, a->vocab, a->logits_dtype, a->logits, a->logits_row_stride, nullptr, 0, &grid);
+        aligned = true;
+        rc = fill_scan(h, A, a->batch, 1, a->vocab, a->logits_dtype, a->logits, a->logits_row_stride, nullptr, 0, 0, &grid);
         if (rc) return rc;
     }
     if (reserve_only) return BORN_OK;
@@ -513,12 +509,12 @@ static int sample_device(Handle* h, const born_sample_args* a_in, cudaStream_t s
         const int64_t rec = kRecordHdrBytes + 8 * (int64_t)a->params.top_k;
         A.mode = kScanLocal;
         A.want_lse = a->out_lse != nullptr;
-        A.out_lse = nullptr;
+        A.out_lse = nullptr;  // (the merge writes it)
         A.packed = h->seg_packed;
         A.packed_row_stride = rec;
         A.packed_seg_stride = rec * a->batch;
         if ((size_t)(rec * a->batch * G) > h->seg_packed_bytes) return fail(h, BORN_ERR_UNSUPPORTED, "batch x segments x top_k exceeds the workspace");
-        if ((rc = launch_scan(h, A, a->logits_dtype, grid, st))) return rc;
+        if ((rc = launch_scan(h, A, a->logits_dtype, aligned, grid, st))) return rc;
         MergeArgs M;
         memset(&M, 0, sizeof M);
         M.gathered = h->seg_packed; M.row_stride = rec; M.seg_stride = rec * a->batch;
@@ -529,7 +525,7 @@ static int sample_device(Handle* h, const born_sample_args* a_in, cudaStream_t s
         M.out_kept_ids = a->out_kept_ids; M.out_kept_count = a->out_kept_count; M.kept_stride = a->kept_stride;
         return launch_merge(h, M, st);
     }
-    return launch_scan(h, A, a->logits_dtype, grid, st);
+    return launch_scan(h, A, a->logits_dtype, aligned, grid, st);
 }
 
 static int sample_check(Handle* h, const born_sample_args* a) {
@@ -874,8 +870,8 @@ int32_t born_debug_expire_wait(void* handle, void* stream) {
     int rc = use_device(h);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    // three tiles of zeros, one row, greedy: three CTAs of one tile each; the middle one's copy is withheld
-    const int V = 3 * (kTileBytes / 4);
+    // twelve blocks of zeros, one row, greedy; one block's copy is withheld
+    const int V = 12 * kBlkTok;
     const size_t bytes = (size_t)V * 4 + 64;
     if ((rc = stage_reserve(h, 15, bytes))) return rc;
     uint8_t* buf = (uint8_t*)h->stage[15].p;
@@ -883,14 +879,14 @@ int32_t born_debug_expire_wait(void* handle, void* stream) {
     ScanArgs A;
     memset(&A, 0, sizeof A);
     int grid = 0;
-    if ((rc = fill_scan(h, A, 1, 1, V, BORN_DTYPE_F32, buf, V, nullptr, 0, &grid))) return rc;
+    if ((rc = fill_scan(h, A, 1, 1, V, BORN_DTYPE_F32, buf, V, nullptr, 0, 0, &grid))) return rc;
     A.params.flags = BORN_FLAG_GREEDY;
     A.out_token = (int32_t*)(buf + (size_t)V * 4);
     A.out_status = (int32_t*)(buf + (size_t)V * 4 + 16);
     A.mode = kScanFull;
     A.timeout_ns = 1000000ull;
-    A.debug_skip_tile = 1;
-    if ((rc = launch_scan(h, A, BORN_DTYPE_F32, grid, st))) return rc;
+    A.debug_skip_blk = 5;
+    if ((rc = launch_scan(h, A, BORN_DTYPE_F32, true, grid, st))) return rc;
     CUDA_TRY(h, cudaStreamSynchronize(st));
     return check_device_error(h);
 }
@@ -1074,7 +1070,8 @@ static int shard_local(Handle* h, const born_shard_args* a, void* packed, bool w
     ScanArgs A;
     memset(&A, 0, sizeof A);
     int grid = 0;
-    int rc = fill_scan(h, A, a->batch, 1, a->vocab_local, a->logits_dtype, a->logits, a->logits_row_stride, nullptr, 0, &grid);
+    const bool aligned = rows_aligned(1, a->vocab_local, a->logits_dtype, a->logits, a->logits_row_stride);
+    int rc = fill_scan(h, A, a->batch, 1, a->vocab_local, a->logits_dtype, a->logits, a->logits_row_stride, nullptr, 0, 0, &grid);
     if (rc) return rc;
     A.params.temperature = a->temperature;
     A.params.top_p = a->top_p;
@@ -1086,7 +1083,7 @@ static int shard_local(Handle* h, const born_shard_args* a, void* packed, bool w
     A.packed = (uint8_t*)packed;
     A.packed_row_stride = born_shard_record_bytes(a->top_k);
     A.packed_seg_stride = 0;
-    return launch_scan(h, A, a->logits_dtype, grid, st);
+    return launch_scan(h, A, a->logits_dtype, aligned, grid, st);
 }
 
 static int shard_merge(Handle* h, const born_shard_args* a, const void* gathered, cudaStream_t st) {
@@ -1142,18 +1139,18 @@ int32_t born_sample_sharded(void* handle, const born_shard_args* a, void* stream
 }  // extern "C"
 
 // ------------------------------------------------------------------ allocation-free entry
-// Scratch for born_sample_static: segment records, mass blocks, row tickets and the device
-// error word in one file-scope array that every GPU loading this library holds until exit.
+// Scratch for born_sample_static: segment records, group keys, mass blocks, row tickets and the
+// device error word in one file-scope array that every GPU loading this library holds until exit.
 namespace {
 constexpr int kStaticMaxBatch = BORN_STATIC_MAX_BATCH;
-constexpr int kStaticRecCap = 512;
-constexpr int kStaticMaxGrid = 512;  // >= two CTAs per SM on any sm_100 part
-constexpr size_t kStaticRecStride = kRecordHdrBytes + (size_t)kStaticRecCap * 8;
-constexpr size_t kStaticRecordsBytes = (size_t)(kStaticMaxBatch + kStaticMaxGrid) * kStaticRecStride;
+constexpr int kStaticRecSlots = 248;  // rows cut into slices: at most this many slices in all
+constexpr size_t kStaticRecordsBytes = (size_t)kStaticRecSlots * (size_t)kSegRecordBytes;
 constexpr size_t kStaticBlocks = BORN_STATIC_MAX_BLOCKS;
 constexpr size_t kStaticBlocksBytes = kStaticBlocks * sizeof(MassBlock);
+constexpr size_t kStaticKeys = (kStaticBlocks / 2 + kStaticMaxBatch) * 32;
+constexpr size_t kStaticKeysBytes = kStaticKeys * sizeof(uint16_t);
 constexpr size_t kStaticTicketsBytes = sizeof(uint32_t) * 2 * kStaticMaxBatch;
-constexpr size_t kStaticBytes = kStaticRecordsBytes + kStaticBlocksBytes + kStaticTicketsBytes + 256;  // (the last 256: error word and counters)
+constexpr size_t kStaticBytes = kStaticRecordsBytes + kStaticBlocksBytes + kStaticKeysBytes + kStaticTicketsBytes + 256;  // (the last 256: error word and counters)
 static_assert(kStaticBytes <= BORN_STATIC_SCRATCH_BYTES, "the header promises at most BORN_STATIC_SCRATCH_BYTES");
 constexpr int kStaticMaxDevices = 64;
 }  // namespace
@@ -1205,16 +1202,16 @@ extern "C" int32_t born_sample_static(const born_sample_args* a, void* stream) {
         h->max_vocab = BORN_MAX_VOCAB;
         h->max_k = BORN_MAX_TOP_K;
         h->num_sms = sms;
-        h->max_grid = 2 * sms < kStaticMaxGrid ? 2 * sms : kStaticMaxGrid;
+        h->max_grid = 2 * sms > kStaticMaxBatch ? 2 * sms : kStaticMaxBatch;  // (never fewer CTAs than rows: no ranges, no records for them)
         h->max_rows = kStaticMaxBatch;
-        h->rec_cap = kStaticRecCap;
-        h->rec_stride = (int64_t)kStaticRecStride;
-        h->records_bytes = kStaticRecordsBytes;
-        h->records = base;
-        h->blocks = reinterpret_cast<MassBlock*>(base + kStaticRecordsBytes);
+        h->rec_slots = kStaticRecSlots;
+        h->blocks = reinterpret_cast<MassBlock*>(base);
         h->blocks_cap = (int64_t)kStaticBlocks;
-        h->tickets = reinterpret_cast<uint32_t*>(base + kStaticRecordsBytes + kStaticBlocksBytes);
-        h->dev_error = reinterpret_cast<int*>(base + kStaticRecordsBytes + kStaticBlocksBytes + kStaticTicketsBytes);
+        h->gkeys = reinterpret_cast<uint16_t*>(base + kStaticBlocksBytes);
+        h->gkeys_cap = (int64_t)kStaticKeys;
+        h->records = base + kStaticBlocksBytes + kStaticKeysBytes;
+        h->tickets = reinterpret_cast<uint32_t*>(base + kStaticBlocksBytes + kStaticKeysBytes + kStaticRecordsBytes);
+        h->dev_error = reinterpret_cast<int*>(base + kStaticBlocksBytes + kStaticKeysBytes + kStaticRecordsBytes + kStaticTicketsBytes);
         g_static_ready[dev] = true;
     }
     // The array keeps whatever the previous call left; the tickets and the error word

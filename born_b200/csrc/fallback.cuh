@@ -1,147 +1,126 @@
-// Exact fallback for rows whose kept set could not be proven to lie inside the complete part
-// of their candidates: top-k above 256, a min-p survivor set or a nucleus beyond the 1024
-// candidates the in-shared-memory selection takes, a candidate buffer that overflowed (rows of
-// equal values), a kept-id list of a whole-vocabulary row.
+// Exact search for rows whose kept set does not fit the 1024 candidates of the in-shared-memory
+// selection: a min-p survivor set or a nucleus of thousands of tokens, rows of equal values, a
+// kept-id list of a whole-vocabulary row, a nucleus over penalised values.
 //
-// It is the sort-free threshold search over the whole row: the row is streamed again (from
-// L2 / HBM, 4096 tokens at a time, penalties and mask applied in shared memory) once per
-// radix digit of the 56-bit rank key (value, -index) -- 12 bits per pass, 4096 bins of exact
-// integer counts and masses in shared memory, the crossing bin found by a block scan -- then
-// once more for the inverse-CDF draw.  Slower than the one-pass route by design (a dozen
-// passes over one row by one CTA), never approximate.  It runs in the CTA that finished the
-// row, after that CTA has streamed its whole tile range, when its shared memory is idle.
+// The kept set is a prefix of the rank order, {rank key >= lowkey}.  The key is found by a threshold
+// search without sorting: one pass over the row sums counts or exact masses in 1024 bins of scaled
+// distance below the maximum, a second one collects the entries of the bin in which the target
+// is crossed, and a radix search over those (at most 1024) gives the exact key; only a bin with more
+// entries than that -- ties -- goes through the digits of the 56-bit rank key one by one.  Another
+// pass sums the kept mass per chunk of the row, and the draw scans the one chunk it falls into.
+// Never approximate.  It runs in the CTA that finished the row, when its ring is idle; the row comes
+// from L2.  A pass takes a warp through the row's blocks: the group keys of a block (where the row
+// still has them) say which of its 32 groups are read at all.
+//
+// What bounds it is the one CTA's issue rate: 0.6 us per pass and 10 000 tokens.  (Before: five passes
+// of 4096 shared-memory bins through a staging buffer and one more with a block scan per 4096
+// tokens; 128256-token rows took 1.0 to 1.2 ms.)
 #pragma once
 #include "scan_common.cuh"
 #include "finish.cuh"
 
 namespace born {
 
-constexpr int kFbChunk = 4096;   // tokens per chunk
-constexpr int kFbBins = 4096;    // bins per radix pass (12 bits)
+constexpr int kFbChunks = 1024;      // chunk sums of the draw
+constexpr int kFbHash = 2048;        // slots of the history table
 
 struct FbCtx {
     const ScanArgs* A;
     ScanShared* sh;
-    float* chunk;                  // kFbChunk logits as the sampler sees them (the buffer in use)
-    float* chunk2[2];              // the two buffers that take turns
-    unsigned long long* hlist;     // distinct history tokens of the row: (count << 32) | token
-    uint32_t* bcnt;                // kFbBins counts
-    unsigned long long* bwt;       // kFbBins masses (also: the masses of one chunk for the draw)
-    int nlist;
-    int b, g, V, id0;
+    const uint8_t* base;             // the row's first logit
+    const uint32_t* mrow;            // the caller row's mask words
+    const uint16_t* gkeys;           // group keys (nullptr: every group counts)
+    uint32_t* limb;                  // [3][kBins]
+    uint32_t* hkeys;                 // history table: keys, then multiplicities
+    uint64_t* sel;                   // kSelCap rank keys
+    unsigned long long* selq;        // kSelCap masses
+    unsigned long long* chunk;       // kFbChunks
+    bool hist;
+    int b, g, V, id0, nb;
     born_row_params rp;
     float m, inv_T;
 };
 
-template <typename T>
-__device__ __forceinline__ float fb_raw(const FbCtx& c, int tok) {
-    const T* row = reinterpret_cast<const T*>(c.A->logits) + (int64_t)c.b * c.A->row_stride + (int64_t)c.g * c.V;
-    if constexpr (sizeof(T) == 4) return __ldg(reinterpret_cast<const float*>(row) + tok);
-    else return bf16_bits_to_f32(__ldg(reinterpret_cast<const uint16_t*>(row) + tok));
-}
-__device__ __forceinline__ bool fb_allowed(const FbCtx& c, int tok) {
-    if (!c.A->mask) return true;
-    const int64_t bi = (int64_t)c.g * c.V + tok;
-    return ((__ldg(c.A->mask + (int64_t)c.b * c.A->mask_stride + (bi >> 5)) >> (bi & 31)) & 1u) != 0;
-}
-
-// Distinct history tokens of the row with their multiplicities (all pairs, once per row).
+// The row's distinct history tokens with their multiplicities, in a hash table.
 __device__ __forceinline__ void fb_history(FbCtx& c) {
     const ScanArgs& A = *c.A;
     const int tid = threadIdx.x;
-    if (tid == 0) c.sh->nl = 0;
+    c.hist = A.history != nullptr && penalties_on(c.rp);
+    if (!c.hist) return;
+    for (int i = tid; i < kFbHash; i += kThreads) { c.hkeys[i] = 0xFFFFFFFFu; c.hkeys[kFbHash + i] = 0u; }
     cta_sync();
-    if (A.history && penalties_on(c.rp)) {
-        int len = A.history_len ? A.history_len[c.b] : A.history_stride;
-        len = max(0, min(min(len, A.history_stride), BORN_MAX_HISTORY));
-        const int32_t* gh = A.history + (int64_t)c.b * A.history_stride;
-        for (int p = tid; p < len; p += kThreads) {
-            const int idg = __ldg(gh + p);
-            const long long tok = (long long)idg - (long long)c.g * c.V;
-            if (tok < 0 || tok >= c.V) continue;
-            int cnt = 0;
-            bool first = true;
-            for (int j = 0; j < len; ++j) {
-                const bool eq = (__ldg(gh + j) == idg);
-                cnt += eq ? 1 : 0;
-                if (eq && j < p) first = false;
-            }
-            if (first) c.hlist[smem_atom_add(&c.sh->nl, 1u)] = ((unsigned long long)cnt << 32) | (uint32_t)tok;
+    int len = A.history_len ? A.history_len[c.b] : A.history_stride;
+    len = max(0, min(min(len, A.history_stride), BORN_MAX_HISTORY));
+    const int32_t* gh = A.history + (int64_t)c.b * A.history_stride;
+    for (int p = tid; p < len; p += kThreads) {
+        const long long tok = (long long)__ldg(gh + p) - (long long)c.g * c.V;
+        if (tok < 0 || tok >= c.V) continue;
+        uint32_t slot = ((uint32_t)tok * 2654435761u) >> 21;
+        for (int probe = 0; probe < kFbHash; ++probe) {
+            const uint32_t old = atomicCAS(&c.hkeys[slot], 0xFFFFFFFFu, (uint32_t)tok);
+            if (old == 0xFFFFFFFFu || old == (uint32_t)tok) { smem_red_add(&c.hkeys[kFbHash + slot], 1u); break; }
+            slot = (slot + 1) & (kFbHash - 1);
         }
     }
     cta_sync();
-    c.nlist = c.sh->nl;
 }
 
-// Chunk ci of the row, as the sampler sees it apart from the penalties: the thread's 16 elements
-// (element tid + 256 * j), into registers.  The loads leave together; nothing waits for them here.
-constexpr int kFbPer = kFbChunk / kThreads;
+// Logit of token `tok` as the sampler sees it.
 template <typename T>
-__device__ __forceinline__ void fb_fetch(const FbCtx& c, int ci, float (&v)[kFbPer]) {
-    const int c0 = ci * kFbChunk;
-    bool ok[kFbPer];
-#pragma unroll
-    for (int j = 0; j < kFbPer; ++j) {
-        const int tok = c0 + (int)threadIdx.x + kThreads * j;
-        ok[j] = tok < c.V && fb_allowed(c, tok);
-    }
-#pragma unroll
-    for (int j = 0; j < kFbPer; ++j) {
-        const int tok = c0 + (int)threadIdx.x + kThreads * j;
-        v[j] = tok < c.V ? fb_raw<T>(c, tok) : -INFINITY;
-    }
-#pragma unroll
-    for (int j = 0; j < kFbPer; ++j)
-        if (!ok[j]) v[j] = -INFINITY;
-}
-// ... from the registers into the buffer whose turn it is, with the history penalties on top.
-template <typename T>
-__device__ __forceinline__ void fb_store(FbCtx& c, int ci, const float (&v)[kFbPer]) {
-    const int tid = threadIdx.x;
-    const int c0 = ci * kFbChunk;
-    c.chunk = c.chunk2[ci & 1];
-#pragma unroll
-    for (int j = 0; j < kFbPer; ++j) c.chunk[tid + kThreads * j] = v[j];
-    cta_sync();  // (also: every thread is done with the chunk before last, whose buffer the next store takes)
-    if (c.nlist > 0) {
-        for (int i = tid; i < c.nlist; i += kThreads) {
-            const unsigned long long e = c.hlist[i];
-            const int tok = (int)(uint32_t)e;
-            if (tok >= c0 && tok < c0 + kFbChunk && fb_allowed(c, tok)) c.chunk[tok - c0] = penalise(c.rp, fb_raw<T>(c, tok), (int)(e >> 32));
+__device__ __forceinline__ float fb_token(const FbCtx& c, int tok) {
+    float z = raw_logit<T>(c.base, tok);
+    if (c.hist) {
+        uint32_t slot = ((uint32_t)tok * 2654435761u) >> 21;
+        for (;;) {
+            const uint32_t key = c.hkeys[slot];
+            if (key == 0xFFFFFFFFu) break;
+            if (key == (uint32_t)tok) { z = penalise(c.rp, z, (int)c.hkeys[kFbHash + slot]); break; }
+            slot = (slot + 1) & (kFbHash - 1);
         }
-        cta_sync();
     }
-}
-template <typename T>
-__device__ __forceinline__ void fb_load(FbCtx& c, int ci) {
-    float v[kFbPer];
-    fb_fetch<T>(c, ci, v);
-    fb_store<T>(c, ci, v);
+    if (c.mrow) {
+        const int64_t bi = (int64_t)c.g * c.V + tok;
+        if (!((__ldg(c.mrow + (bi >> 5)) >> (bi & 31)) & 1u)) z = -INFINITY;
+    }
+    return z;
 }
 
-// One pass over the row: f(token, z) for every token above -inf, by the thread that owns it.  The
-// next chunk's loads are in flight while the current chunk is worked on.
+// One block of 1024 tokens by the warp: f(tok, z) with eight groups at a time, a lane per token
+// (z = -inf where there is none).  Groups whose key is below `low16` are not read.
 template <typename T, typename F>
-__device__ __forceinline__ void fb_pass(FbCtx& c, F f) {
-    const int nchunks = (c.V + kFbChunk - 1) / kFbChunk;
-    float v[kFbPer];
-    fb_fetch<T>(c, 0, v);
-    for (int ci = 0; ci < nchunks; ++ci) {
-        fb_store<T>(c, ci, v);
-        if (ci + 1 < nchunks) fb_fetch<T>(c, ci + 1, v);
-        const float* ch = c.chunk;
-        for (int e = threadIdx.x; e < kFbChunk; e += kThreads) {
-            const float z = ch[e];
-            if (z > -INFINITY) f(ci * kFbChunk + e, z);
+__device__ __forceinline__ void fb_block(const FbCtx& c, int j, uint32_t low16, F f) {
+    const int lane = threadIdx.x & 31;
+    const int ngrp = (c.V + kGrpTok - 1) / kGrpTok;
+    const int gi = j * 32 + lane;
+    const uint32_t key = gi < ngrp ? (c.gkeys ? (uint32_t)c.gkeys[gi] : 0xFFFFu) : 0u;
+    uint32_t hb = __ballot_sync(0xffffffffu, key >= low16 && gi < ngrp);
+    while (hb) {
+        int tok[8];
+        float z[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            tok[e] = hb ? (j * 32 + __ffs(hb) - 1) * kGrpTok + lane : c.V;
+            hb &= hb - 1;
         }
+        if (!c.hist && !c.mrow) {  // (the loads leave together)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) z[e] = tok[e] < c.V ? raw_logit<T>(c.base, tok[e]) : -INFINITY;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) z[e] = tok[e] < c.V ? fb_token<T>(c, tok[e]) : -INFINITY;
+        }
+        f(tok, z);
     }
+}
+// One pass over the row; ends on a barrier.
+template <typename T, typename F>
+__device__ __forceinline__ void fb_pass(const FbCtx& c, uint32_t low16, F f) {
+    for (int j = threadIdx.x >> 5; j < c.nb; j += kScanWarps) fb_block<T>(c, j, low16, f);
     cta_sync();
 }
 
-__device__ __forceinline__ unsigned long long fb_mass(const FbCtx& c, float z) {
-    const float x = scaled_shift(z, c.m, c.inv_T);
-    return (x < -30.0f) ? 0ull : mass_of(x);
-}
+__device__ __forceinline__ unsigned long long fb_mass(const FbCtx& c, float z) { return mass_of(scaled_shift(z, c.m, c.inv_T)); }
+__device__ __forceinline__ uint32_t fb_low16(unsigned long long lowkey) { return (uint32_t)(lowkey >> 40); }
 
 // Walking the tokens with rank key >= lowkey in rank order (key descending), the key at which the
 // running weight (1 per token, or its mass) first exceeds `target`.  Returns 0 when the total
@@ -150,143 +129,167 @@ template <typename T, bool kWeighted>
 __device__ __noinline__ unsigned long long fb_search(FbCtx& c, unsigned long long lowkey, unsigned long long target) {
     const int tid = threadIdx.x;
     ScanShared& sh = *c.sh;
-    unsigned long long prefix = 0, pmask = 0;
-    const int shifts[5] = {44, 32, 20, 8, 0};
-    // Masses are summed per bin as three 14-bit limbs in 32-bit words: 32-bit shared-memory atomics
-    // are native, 64-bit ones are compare-and-swap loops.  A limb sum stays below 2^32 for rows of
-    // up to 2^17 tokens; longer rows use the 64-bit words.
-    uint32_t* limb = reinterpret_cast<uint32_t*>(c.bwt);  // [3][kFbBins], over the mass and count areas
-    const bool limbs = kWeighted && c.V <= (1 << 17);
-    for (int lvl = 0; lvl < 5; ++lvl) {
-        const int shift = shifts[lvl];
-        const int nb = (lvl == 4) ? 256 : kFbBins;
-        if (limbs) {
-            for (int i = tid; i < 3 * kFbBins; i += kThreads) limb[i] = 0;
-        } else {
-            for (int i = tid; i < nb; i += kThreads) { c.bcnt[i] = 0; c.bwt[i] = 0; }
-        }
+    uint32_t* limb = c.limb;
+    const uint32_t low16 = fb_low16(lowkey);
+    auto clear = [&]() {
+        for (int i = tid; i < 3 * kBins / 4; i += kThreads) reinterpret_cast<uint4*>(limb)[i] = make_uint4(0u, 0u, 0u, 0u);
         cta_sync();
-        fb_pass<T>(c, [&](int tok, float z) {
-            const unsigned long long ck = make_ck(z, c.id0 + tok);
-            if (ck < lowkey || (ck & pmask) != prefix) return;
-            const uint32_t d = (uint32_t)(ck >> shift) & (uint32_t)(nb - 1);
-            if (kWeighted) {
-                const unsigned long long w = fb_mass(c, z);
-                if (!w) return;
-                if (limbs) {
-                    smem_red_add(&limb[d], (uint32_t)w & 0x3FFFu);
-                    smem_red_add(&limb[kFbBins + d], (uint32_t)(w >> 14) & 0x3FFFu);
-                    smem_red_add(&limb[2 * kFbBins + d], (uint32_t)(w >> 28));
-                } else {
-                    atomicAdd(&c.bwt[d], w);
+    };
+    auto total_of = [&](int i) { return kWeighted ? bin_total(limb, i) : (uint64_t)limb[i]; };
+    unsigned long long before = 0;
+    int bin = -1;
+    // (three 14-bit limbs hold the masses of 2^18 tokens; longer rows go digit by digit, in 64-bit words)
+    const bool wide = kWeighted && c.V > (1 << 18);
+    if (!wide) {
+        clear();
+        fb_pass<T>(c, low16, [&](const int (&tok)[8], const float (&z)[8]) {
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+                uint64_t q[2] = {1, 1};
+                if (kWeighted) mass2_of(make_float2(z[e], z[e + 1]), c.m, c.inv_T, q[0], q[1]);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (!(z[e + h] > -INFINITY) || make_ck(z[e + h], c.id0 + tok[e + h]) < lowkey) continue;
+                    const int bn = nucleus_bin(z[e + h], c.m, c.inv_T);
+                    if (kWeighted) bin_mass(limb, bn, q[h]);
+                    else smem_red_add(&limb[bn], 1u);
                 }
-            } else {
-                smem_red_add(&c.bcnt[d], 1u);
             }
         });
-        if (limbs) {  // fold the limbs into the 64-bit words the scan below reads
-            unsigned long long w[kFbBins / kThreads];
+        bin = find_bin(total_of, target, before, sh);
+        if (bin < 0) return 0ull;
+        target -= before;
+        // the entries of the crossing bin
+        if (tid == 0) sh.nl = 0;
+        cta_sync();
+        fb_pass<T>(c, low16, [&](const int (&tok)[8], const float (&z)[8]) {
 #pragma unroll
-            for (int j = 0; j < kFbBins / kThreads; ++j) {
-                const int bin = tid + kThreads * j;
-                w[j] = (unsigned long long)limb[bin] + ((unsigned long long)limb[kFbBins + bin] << 14) +
-                       ((unsigned long long)limb[2 * kFbBins + bin] << 28);
+            for (int e = 0; e < 8; ++e) {
+                const unsigned long long ck = make_ck(z[e], c.id0 + tok[e]);
+                if (!(z[e] > -INFINITY) || ck < lowkey || nucleus_bin(z[e], c.m, c.inv_T) != bin) continue;
+                const uint32_t pos = smem_atom_add(&sh.nl, 1u);
+                if (pos < (uint32_t)kSelCap) { c.sel[pos] = ck; c.selq[pos] = kWeighted ? fb_mass(c, z[e]) : 1ull; }
             }
-            cta_sync();
-#pragma unroll
-            for (int j = 0; j < kFbBins / kThreads; ++j) c.bwt[tid + kThreads * j] = w[j];
-            cta_sync();
-        }
-        // block scan over the bins in walk order (descending digit): thread t owns nb/256 of them
-        const int per = nb / kThreads;
-        unsigned long long loc = 0;
-        for (int j = 0; j < per; ++j) {
-            const int bin = nb - 1 - (tid * per + j);
-            loc += kWeighted ? c.bwt[bin] : (unsigned long long)c.bcnt[bin];
-        }
-        unsigned long long incl = loc;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const unsigned long long up = shfl_up_u64(incl, d);
-            if ((tid & 31) >= d) incl += up;
-        }
-        cta_sync();
-        if ((tid & 31) == 31) sh.red64[tid >> 5] = incl;
-        if (tid == 0) sh.found = -1;
-        cta_sync();
-        unsigned long long off = 0, total = 0;
-#pragma unroll
-        for (int w = 0; w < kScanWarps; ++w) {
-            const unsigned long long x = sh.red64[w];
-            if (w < (tid >> 5)) off += x;
-            total += x;
-        }
-        incl += off;
-        if (total <= target) return 0ull;  // (uniform)
-        if (incl > target && incl - loc <= target) {
-            unsigned long long acc = incl - loc;
-            for (int j = 0; j < per; ++j) {
-                const int bin = nb - 1 - (tid * per + j);
-                const unsigned long long w = kWeighted ? c.bwt[bin] : (unsigned long long)c.bcnt[bin];
-                if (acc + w > target) { sh.found = bin; sh.before = acc; break; }
-                acc += w;
-            }
-        }
-        cta_sync();
-        const unsigned long long digit = (unsigned long long)sh.found;
-        target -= sh.before;
-        prefix |= digit << shift;
-        pmask |= (unsigned long long)(nb - 1) << shift;
-        cta_sync();
+        });
+        const int n = sh.nl;
+        if (n <= kSelCap)
+            return block_radix_search<true, 56, !kWeighted>(
+                n, target, [&](int i) { return c.sel[i]; }, [&](int i) { return c.selq[i]; }, sh.sc);
     }
-    return prefix;
+    // more entries than that in one bin: ten bits of the rank key per pass
+    unsigned long long prefix = 0, pmask = 0;
+    unsigned long long* wide_bins = c.selq;  // kBins 64-bit words, when limbs could overflow
+    for (int shift = 46;; shift = shift > 10 ? shift - 10 : 0) {
+        clear();
+        if (wide) {
+            for (int i = tid; i < kBins; i += kThreads) wide_bins[i] = 0;
+            cta_sync();
+        }
+        fb_pass<T>(c, low16, [&](const int (&tok)[8], const float (&z)[8]) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const unsigned long long ck = make_ck(z[e], c.id0 + tok[e]);
+                if (!(z[e] > -INFINITY) || ck < lowkey || (ck & pmask) != prefix) continue;
+                if (!wide && nucleus_bin(z[e], c.m, c.inv_T) != bin) continue;
+                const int d = (int)((ck >> shift) & (unsigned long long)(kBins - 1));
+                if (!kWeighted) smem_red_add(&limb[d], 1u);
+                else if (wide) atomicAdd(&wide_bins[d], fb_mass(c, z[e]));
+                else bin_mass(limb, d, fb_mass(c, z[e]));
+            }
+        });
+        // (walk order is descending digit)
+        const int o = find_bin([&](int i) { return wide ? (uint64_t)wide_bins[kBins - 1 - i] : total_of(kBins - 1 - i); }, target, before, sh);
+        if (o < 0) return 0ull;
+        target -= before;
+        prefix |= (unsigned long long)(kBins - 1 - o) << shift;
+        pmask |= (unsigned long long)(kBins - 1) << shift;
+        prefix &= pmask;
+        cta_sync();
+        if (shift == 0) return prefix;
+    }
 }
 
-// The (at most kSelCap) tokens with rank key >= lowkey, gathered and written in rank order.
+// The (at most kSelCap) tokens with rank key >= lowkey, in sel.
 template <typename T>
-__device__ __forceinline__ int fb_gather(FbCtx& c, unsigned long long lowkey, uint64_t* sel) {
+__device__ __forceinline__ int fb_gather(FbCtx& c, unsigned long long lowkey) {
+    cta_sync();
     if (threadIdx.x == 0) c.sh->nl = 0;
     cta_sync();
-    fb_pass<T>(c, [&](int tok, float z) {
-        const unsigned long long ck = make_ck(z, c.id0 + tok);
-        if (ck >= lowkey) {
-            const int pos = (int)smem_atom_add(&c.sh->nl, 1u);
-            if (pos < kSelCap) sel[pos] = ck;
+    fb_pass<T>(c, fb_low16(lowkey), [&](const int (&tok)[8], const float (&z)[8]) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const unsigned long long ck = make_ck(z[e], c.id0 + tok[e]);
+            if (!(z[e] > -INFINITY) || ck < lowkey) continue;
+            const uint32_t pos = smem_atom_add(&c.sh->nl, 1u);
+            if (pos < (uint32_t)kSelCap) c.sel[pos] = ck;
         }
     });
     return min(c.sh->nl, kSelCap);
 }
 
+// The `count` first tokens in rank order of {rank key >= lowkey}, into the caller's kept-id list.
+template <typename T>
+__device__ __forceinline__ void fb_kept_ids(FbCtx& c, unsigned long long lowkey, int count) {
+    const ScanArgs& A = *c.A;
+    unsigned long long Cr = fb_search<T, false>(c, lowkey, (unsigned long long)(count - 1));
+    if (Cr < lowkey) Cr = lowkey;
+    const int n = fb_gather<T>(c, Cr);
+    for (int i = threadIdx.x; i < n; i += kThreads) {
+        int rank = 0;
+        for (int j = 0; j < n; ++j) rank += (c.sel[j] > c.sel[i]) ? 1 : 0;
+        if (rank < A.kept_stride) A.out_kept_ids[(int64_t)c.b * A.kept_stride + rank] = ck_idx(c.sel[i]);
+    }
+    cta_sync();
+}
+
 template <typename T>
 __device__ __noinline__ void fallback_row(const ScanArgs& A, ScanShared& sh, uint8_t* smem, int row) {
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     FbCtx c;
     c.A = &A;
     c.sh = &sh;
-    // 88 KB of the CTA's dynamic shared memory (no variant of the kernel has less):
-    // two chunk buffers | history list | mass bins | count bins
-    c.chunk2[0] = reinterpret_cast<float*>(smem);
-    c.chunk2[1] = reinterpret_cast<float*>(smem + kFbChunk * 4);
-    c.chunk = c.chunk2[0];
-    c.hlist = reinterpret_cast<unsigned long long*>(smem + 2 * kFbChunk * 4);
-    c.bwt = reinterpret_cast<unsigned long long*>(smem + 2 * kFbChunk * 4 + BORN_MAX_HISTORY * 8);
-    c.bcnt = reinterpret_cast<uint32_t*>(smem + 2 * kFbChunk * 4 + BORN_MAX_HISTORY * 8 + kFbBins * 8);
-    static_assert(2 * kFbChunk * 4 + BORN_MAX_HISTORY * 8 + kFbBins * 12 <= kScanStages * kTileBytes + kScanWarps * kWarpCand * 8 + kSelCap * 8,
-                  "the exact search lives in the streaming kernel's shared memory");
-    uint64_t* sel = reinterpret_cast<uint64_t*>(c.bwt);  // gathers happen when no search is in flight
+    // (kExactBytes of the CTA's dynamic shared memory)
+    c.limb = reinterpret_cast<uint32_t*>(smem);
+    c.hkeys = c.limb + 3 * kBins;
+    c.sel = reinterpret_cast<uint64_t*>(c.hkeys + 2 * kFbHash);
+    c.selq = reinterpret_cast<unsigned long long*>(c.sel + kSelCap);
+    c.chunk = c.selq + kSelCap;
+    static_assert(3 * kBins * 4 + 2 * kFbHash * 4 + 2 * kSelCap * 8 + kFbChunks * 8 <= kExactBytes, "the exact search's shared memory");
     c.b = row / A.G;
     c.g = row - c.b * A.G;
     c.V = A.V;
+    c.nb = A.nb;
     c.id0 = A.idx_base + c.g * A.V;
     c.rp = A.row_params ? A.row_params[c.b] : A.params;
+    c.base = row_geom<T>(A, row).base;
+    c.mrow = A.mask ? A.mask + (int64_t)c.b * A.mask_stride : nullptr;
     const RowPlan pl = row_plan(c.rp);
     c.inv_T = pl.inv_T;
     fb_history(c);
+    // Group keys: still there when the row has a CTA or more to itself (a CTA that streams many rows
+    // re-uses their place).  bf16 rows with penalties have history tokens that are not in them.
+    c.gkeys = nullptr;
+    if (A.slices > 0 && (!pl.need_mass || pl.window) && !(sizeof(T) == 2 && c.hist))
+        c.gkeys = A.slices == 1 && c.nb * 32 <= A.L.gkeys_cap ? reinterpret_cast<const uint16_t*>(smem + A.L.gkeys) : A.gkeys + (int64_t)row * (c.nb * 32);
 
-    // row maximum (the row is known to be valid: the finish only defers rows with a finite maximum)
-    float mx = -INFINITY;
-    fb_pass<T>(c, [&](int, float z) { mx = fmaxf(mx, z); });
-    c.m = block_max_nan(mx, sh.redf);
+    // row maximum (the row is known to be valid: only rows with a finite maximum get here)
+    {
+        uint32_t top16 = 0;
+        if (c.gkeys) {  // only the groups that share the best key
+            for (int i = tid; i < c.nb * 32; i += kThreads) top16 = max(top16, (uint32_t)c.gkeys[i]);
+            top16 = __reduce_max_sync(0xffffffffu, top16);
+            if (lane == 0) sh.redu[warp] = top16;
+            cta_sync();
+#pragma unroll
+            for (int w = 0; w < kScanWarps; ++w) top16 = max(top16, sh.redu[w]);
+        }
+        float mx = -INFINITY;
+        fb_pass<T>(c, top16, [&](const int (&)[8], const float (&z)[8]) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) mx = fmaxf(mx, z[e]);
+        });
+        c.m = block_max(mx, sh.redf);
+    }
 
     RowOut o;
     o.token = A.out_token; o.prob = A.out_prob; o.lse = A.out_lse; o.status = A.out_status;
@@ -295,30 +298,35 @@ __device__ __noinline__ void fallback_row(const ScanArgs& A, ScanShared& sh, uin
     const unsigned long long alive = 1ull << 24;  // smallest rank key of a token above -inf
 
     if (A.mode == kScanLocal) {
-        // the k best of the virtual row, in rank order
+        // the k best of the virtual row, in rank order; the record's sum of 2^((z - m) * c2) with them
         unsigned long long Ck = fb_search<T, false>(c, alive, (unsigned long long)(pl.k - 1));
         if (Ck == 0) Ck = alive;
-        const int n = fb_gather<T>(c, Ck, sel);
-        // statistics of the record come from the segment headers
-        const int c_first = cta_of_tile((long long)row * A.tpr, (long long)A.B * A.G * A.tpr, gridDim.x);
-        const int c_last = cta_of_tile((long long)(row + 1) * A.tpr - 1, (long long)A.B * A.G * A.tpr, gridDim.x);
         float ls = 0.0f;
-        for (int s = tid; s <= c_last - c_first; s += kThreads) {
-            const float4 h = __ldcg(reinterpret_cast<const float4*>(A.records + (int64_t)(row + c_first + s) * A.rec_stride));
-            if (h.y > 0.0f) ls += h.y * ex2_approx(__fmul_rn(h.x - c.m, pl.c2));
-        }
-        ls = block_sum_f32(ls, sh.redf);
-        write_packed(A, sh, sel, reinterpret_cast<unsigned long long*>(sel + kSelCap), n, pl.k, c.b, c.g, c.m, ls, -INFINITY, true);
+        fb_pass<T>(c, 0u, [&](const int (&)[8], const float (&z)[8]) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) ls += ex2_approx(__fmul_rn(z[e] - c.m, pl.c2));
+        });
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, d);
+        if (lane == 0) sh.redf[warp] = ls;
+        const int n = fb_gather<T>(c, Ck);
+        ls = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kScanWarps; ++w) ls += sh.redf[w];
+        write_packed(A, sh, c.sel, reinterpret_cast<uint64_t*>(c.selq), n, pl.k, c.b, c.g, c.m, ls);
         return;
     }
 
     if (pl.greedy) {
         uint64_t best = 0;
-        fb_pass<T>(c, [&](int tok, float z) { best = max(best, make_ck(z, c.id0 + tok)); });
+        fb_pass<T>(c, zkey(c.m) >> 16, [&](const int (&tok)[8], const float (&z)[8]) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if (z[e] >= c.m) best = max(best, make_ck(z[e], c.id0 + tok[e]));
+        });
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) best = max(best, shfl_xor_u64(best, d));
-        cta_sync();
-        if ((tid & 31) == 0) sh.red64[tid >> 5] = best;
+        if (lane == 0) sh.red64[warp] = best;
         cta_sync();
         if (tid == 0) {
             for (int w = 1; w < kScanWarps; ++w) best = max(best, (uint64_t)sh.red64[w]);
@@ -338,20 +346,29 @@ __device__ __noinline__ void fallback_row(const ScanArgs& A, ScanShared& sh, uin
         const unsigned long long Ck = fb_search<T, false>(c, lowkey, (unsigned long long)(pl.k - 1));
         if (Ck > lowkey) lowkey = Ck;
     }
-    if (c.rp.min_p > 0.0f) {
+    if (pl.minp) {
         // the survivors are a prefix of the rank order (masses fall with the value): lowest surviving value
         const unsigned long long Qa = __double2ull_ru((double)c.rp.min_p * 1099511627776.0);
+        const unsigned long long near_cut = (unsigned long long)zkey(c.m + pl.delta) << 24;
         uint32_t zmin = 0xFFFFFFFFu;
-        fb_pass<T>(c, [&](int tok, float z) {
-            if (make_ck(z, c.id0 + tok) >= lowkey && fb_mass(c, z) >= Qa) zmin = min(zmin, zkey(z));
+        fb_pass<T>(c, fb_low16(max(lowkey, near_cut)), [&](const int (&tok)[8], const float (&z)[8]) {
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+                uint64_t q[2];
+                mass2_of(make_float2(z[e], z[e + 1]), c.m, c.inv_T, q[0], q[1]);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (z[e + h] > -INFINITY && q[h] >= Qa && make_ck(z[e + h], c.id0 + tok[e + h]) >= lowkey) zmin = min(zmin, zkey(z[e + h]));
+            }
         });
         zmin = __reduce_min_sync(0xffffffffu, zmin);
+        if (lane == 0) sh.redu[warp] = zmin;
         cta_sync();
-        if ((tid & 31) == 0) sh.red64[tid >> 5] = zmin;
-        cta_sync();
-        for (int w = 0; w < kScanWarps; ++w) zmin = min(zmin, (uint32_t)sh.red64[w]);
+#pragma unroll
+        for (int w = 0; w < kScanWarps; ++w) zmin = min(zmin, sh.redu[w]);
         const unsigned long long Cm = (unsigned long long)zmin << 24;
         if (Cm > lowkey) lowkey = Cm;
+        cta_sync();
     }
     unsigned long long S_tot = 0;
     if (pl.need_mass) {
@@ -362,27 +379,23 @@ __device__ __noinline__ void fallback_row(const ScanArgs& A, ScanShared& sh, uin
     }
     if (pl.need_mass && !pl.window) {
         // whole-row draw; only the kept-id list brought the row here
-        if (A.out_kept_ids) {
-            const int R = min(A.kept_stride, kSelCap);
-            unsigned long long Cr = fb_search<T, false>(c, alive, (unsigned long long)(R - 1));
-            if (Cr == 0) Cr = alive;
-            const int n = fb_gather<T>(c, Cr, sel);
-            for (int i = tid; i < n; i += kThreads) {
-                int rank = 0;
-                for (int j = 0; j < n; ++j) rank += (sel[j] > sel[i]) ? 1 : 0;
-                if (rank < A.kept_stride) A.out_kept_ids[(int64_t)c.b * A.kept_stride + rank] = ck_idx(sel[i]);
-            }
-            cta_sync();
-        }
-        draw_whole_row<T>(A, sh, smem, o, c.rp, c.b, c.g, row, c.m, pl.inv_T, S_tot, u);
+        if (A.out_kept_ids) fb_kept_ids<T>(c, alive, min(A.kept_stride, kSelCap));
+        draw_whole_row<T>(A, sh, o, c.rp, c.b, c.g, row, c.m, pl.inv_T, S_tot, u);
         return;
     }
-    if (c.rp.top_p > 0.0f && c.rp.top_p < 1.0f) {
+    if (pl.topp) {
         unsigned long long S = S_tot;
         if (!pl.need_mass) {
             unsigned long long part = 0;
-            fb_pass<T>(c, [&](int tok, float z) {
-                if (make_ck(z, c.id0 + tok) >= lowkey) part += fb_mass(c, z);
+            fb_pass<T>(c, fb_low16(lowkey), [&](const int (&tok)[8], const float (&z)[8]) {
+#pragma unroll
+                for (int e = 0; e < 8; e += 2) {
+                    uint64_t q[2];
+                    mass2_of(make_float2(z[e], z[e + 1]), c.m, c.inv_T, q[0], q[1]);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        if (make_ck(z[e + h], c.id0 + tok[e + h]) >= lowkey) part += q[h];
+                }
             });
             S = block_sum_u64(part, sh.red64);
         }
@@ -391,84 +404,85 @@ __device__ __noinline__ void fallback_row(const ScanArgs& A, ScanShared& sh, uin
         const unsigned long long Cp = fb_search<T, true>(c, lowkey, Tp - 1);
         if (Cp > lowkey) lowkey = Cp;
     }
-    // the kept set is {rank key >= lowkey}: its mass, its size, then the draw in ascending token index
-    unsigned long long part = 0;
+    // the kept set is {rank key >= lowkey}: its mass per chunk of the row, and its size
+    int cl = 0;  // blocks per chunk, as a shift
+    while (((c.nb - 1) >> cl) >= kFbChunks) ++cl;
+    const int nchunk = ((c.nb - 1) >> cl) + 1;
     int cnt = 0;
-    fb_pass<T>(c, [&](int tok, float z) {
-        if (make_ck(z, c.id0 + tok) >= lowkey) { part += fb_mass(c, z); ++cnt; }
-    });
+    cta_sync();
+    for (int ch = warp; ch < nchunk; ch += kScanWarps) {
+        unsigned long long part = 0;
+        for (int j = ch << cl; j < min(c.nb, (ch + 1) << cl); ++j)
+            fb_block<T>(c, j, fb_low16(lowkey), [&](const int (&tok)[8], const float (&z)[8]) {
+#pragma unroll
+                for (int e = 0; e < 8; e += 2) {
+                    uint64_t q[2];
+                    mass2_of(make_float2(z[e], z[e + 1]), c.m, c.inv_T, q[0], q[1]);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        if (z[e + h] > -INFINITY && make_ck(z[e + h], c.id0 + tok[e + h]) >= lowkey) { part += q[h]; ++cnt; }
+                }
+            });
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) part += shfl_xor_u64(part, d);
+        if (lane == 0) c.chunk[ch] = part;
+    }
+    const int n_kept = (int)block_sum_u64((uint64_t)cnt, sh.red64);  // (its barriers cover the chunk sums)
+    unsigned long long part = 0;
+    for (int ch = tid; ch < nchunk; ch += kThreads) part += c.chunk[ch];
     const unsigned long long S = block_sum_u64(part, sh.red64);
-    const int n_kept = (int)block_sum_u64((uint64_t)cnt, sh.red64);
     if (S == 0) {
         row_fail(o, BORN_ROW_ALL_MASKED);
         return;
     }
     unsigned long long t = __double2ull_rz(__dmul_rn((double)u, __ull2double_rn(S)));
     if (t > S - 1) t = S - 1;
-    {
-        unsigned long long run = 0;
-        const int nchunks = (c.V + kFbChunk - 1) / kFbChunk;
-        unsigned long long* qm = c.bwt;  // masses of one chunk, in token order
-        for (int ci = 0; ci < nchunks; ++ci) {
-            fb_load<T>(c, ci);
-            for (int e = tid; e < kFbChunk; e += kThreads) {
-                const float z = c.chunk[e];
-                qm[e] = (z > -INFINITY && make_ck(z, c.id0 + ci * kFbChunk + e) >= lowkey) ? fb_mass(c, z) : 0ull;
-            }
-            cta_sync();
-            constexpr int PER = kFbChunk / kThreads;  // consecutive tokens per thread
-            unsigned long long loc = 0;
-            for (int j = 0; j < PER; ++j) loc += qm[tid * PER + j];
-            unsigned long long incl = loc;
+    unsigned long long before;
+    cta_sync();
+    const int ch = find_bin([&](int i) { return i < nchunk ? (uint64_t)c.chunk[i] : 0ull; }, t, before, sh);
+    t -= before;
+    // inside the chunk: four consecutive tokens per thread, block by block
+    for (int j = ch << cl; j < min(c.nb, (ch + 1) << cl); ++j) {
+        const int tok0 = j * kBlkTok + 4 * tid;
+        uint64_t q[4] = {0, 0, 0, 0};
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const unsigned long long up = shfl_up_u64(incl, d);
-                if ((tid & 31) >= d) incl += up;
-            }
-            cta_sync();
-            if ((tid & 31) == 31) sh.red64[tid >> 5] = incl;
-            cta_sync();
-            unsigned long long off = 0, total = 0;
+        for (int i = 0; i < 4; ++i) {
+            if (tok0 + i >= c.V) continue;
+            const float z = fb_token<T>(c, tok0 + i);
+            if (z > -INFINITY && make_ck(z, c.id0 + tok0 + i) >= lowkey) q[i] = fb_mass(c, z);
+        }
+        const uint64_t loc = q[0] + q[1] + q[2] + q[3];
+        uint64_t incl = loc;
 #pragma unroll
-            for (int w = 0; w < kScanWarps; ++w) {
-                const unsigned long long x = sh.red64[w];
-                if (w < (tid >> 5)) off += x;
-                total += x;
-            }
-            incl += off;
-            if (run + total > t) {  // the token is in this chunk (uniform)
-                if (run + incl > t && run + incl - loc <= t) {
-                    unsigned long long acc = run + incl - loc;
-                    for (int j = 0; j < PER; ++j) {
-                        const unsigned long long q = qm[tid * PER + j];
-                        if (acc + q > t) {
-                            A.out_token[c.b] = c.id0 + ci * kFbChunk + tid * PER + j;
-                            A.out_status[c.b] = BORN_ROW_OK;
-                            if (A.out_prob) A.out_prob[c.b] = __double2float_rn(__ddiv_rn(__ull2double_rn(q), __ull2double_rn(S)));
-                            break;
-                        }
-                        acc += q;
-                    }
-                }
-                break;
-            }
-            run += total;
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint64_t up = shfl_up_u64(incl, d);
+            if (lane >= d) incl += up;
         }
         cta_sync();
+        if (lane == 31) sh.red64[warp] = incl;
+        cta_sync();
+        uint64_t total = 0;
+#pragma unroll
+        for (int w = 0; w < kScanWarps; ++w) {
+            const uint64_t x = sh.red64[w];
+            if (w < warp) incl += x;
+            total += x;
+        }
+        if (total > t) {  // (uniform)
+            if (incl > t && incl - loc <= t) {
+                uint64_t acc = incl - loc;
+                int i = 0;
+                for (; i < 3 && acc + q[i] <= t; ++i) acc += q[i];
+                A.out_token[c.b] = c.id0 + tok0 + i;
+                A.out_status[c.b] = BORN_ROW_OK;
+                if (A.out_prob) A.out_prob[c.b] = __double2float_rn(__ddiv_rn(__ull2double_rn(q[i]), __ull2double_rn(S)));
+            }
+            break;
+        }
+        t -= total;
     }
     if (A.out_kept_count && tid == 0) A.out_kept_count[c.b] = n_kept;
-    if (A.out_kept_ids) {
-        const int R = min(min(A.kept_stride, kSelCap), n_kept);
-        unsigned long long Cr = fb_search<T, false>(c, lowkey, (unsigned long long)(R - 1));
-        if (Cr < lowkey) Cr = lowkey;
-        const int n = fb_gather<T>(c, Cr, sel);
-        for (int i = tid; i < n; i += kThreads) {
-            int rank = 0;
-            for (int j = 0; j < n; ++j) rank += (sel[j] > sel[i]) ? 1 : 0;
-            if (rank < A.kept_stride) A.out_kept_ids[(int64_t)c.b * A.kept_stride + rank] = ck_idx(sel[i]);
-        }
-        cta_sync();
-    }
+    if (A.out_kept_ids) fb_kept_ids<T>(c, lowkey, min(min(A.kept_stride, kSelCap), n_kept));
 }
 
 }  // namespace born

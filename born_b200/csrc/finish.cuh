@@ -1,12 +1,16 @@
-// Finishing a row: merge the segment records, select (top-k -> min-p -> top-p on exact
+// Finishing a row: fold the segments' statistics, work out from the group keys which groups of 32
+// tokens can hold tokens that matter, read those again, select (top-k -> min-p -> top-p on exact
 // integer masses) and draw by inverse CDF in ascending token index.  Runs in the CTA that
-// completes the row (scan_kernel) or in merge_kernel over all-gathered shard records.
+// completes the row (scan_kernel) or, from the selection on, in merge_kernel over all-gathered
+// shard records.
 //
 // Every decision sum is an exact integer sum of fixed-point masses
 // q = rne(exp_det((z - m) * inv_T) * 2^40), so thread order cannot matter.  Rank order is
 // (value descending, token index ascending): the first maximum wins, as in the reference's
 // argmax (born: internal/nn/cross_entropy.go:241-251).
 #pragma once
+#include <float.h>
+#include <string.h>
 #include "scan_common.cuh"
 
 namespace born {
@@ -41,7 +45,6 @@ struct SelectIn {
     unsigned long long Qa;     // min-p threshold on the masses (0: off)
     float top_p;    // (0,1): on
     unsigned long long S_ext;  // top-p total when the candidates are only the heavy part of the row (0: their own sum)
-    bool complete;  // the candidates hold every token the row can keep
     float m_row, inv_T, u;
 };
 
@@ -50,9 +53,8 @@ struct SelectIn {
 // number of larger keys (keys are unique: the token index is part of them); candidates and
 // masses are then re-written in rank order, and since a mass never grows along that order the
 // kept set of every filter is a prefix of it, which every thread finds by walking the sorted
-// masses itself.  Returns false when the nucleus is not inside the candidates (the caller then
-// takes the exact fallback); all threads get the same answer.
-__device__ __forceinline__ bool select_small(const SelectIn& in, uint64_t* sel, unsigned long long* selq, ScanShared& sh,
+// masses itself.
+__device__ __forceinline__ void select_small(const SelectIn& in, uint64_t* sel, unsigned long long* selq, ScanShared& sh,
                                              const RowOut& o) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = in.n;
@@ -118,10 +120,9 @@ __device__ __forceinline__ bool select_small(const SelectIn& in, uint64_t* sel, 
     cta_sync();
     const int R = sh.nw;
     const uint64_t S = sh.acc[0];
-    if (topp && in.S_ext && !in.complete && S < Tp) return false;  // (uniform)
     if (S == 0) {  // cannot happen while the row maximum is finite; never divide by it
         row_fail(o, BORN_ROW_ALL_MASKED);
-        return true;
+        return;
     }
     uint64_t t = __double2ull_rz(__dmul_rn((double)in.u, __ull2double_rn(S)));
     if (t > S - 1) t = S - 1;
@@ -145,12 +146,11 @@ __device__ __forceinline__ bool select_small(const SelectIn& in, uint64_t* sel, 
         if (o.kept_ids && tid < o.kept_stride) o.kept_ids[(int64_t)o.row * o.kept_stride + tid] = ck_idx(c2);
     }
     if (o.kept_count && tid == 0) o.kept_count[o.row] = R;
-    return true;
 }
 
 // Selection and draw over kThreads < n <= kSelCap candidates: radix select, then mass-weighted
-// radix threshold searches.  Same rules, same answer convention as select_small.
-static __device__ __noinline__ bool select_and_draw(const SelectIn in, uint64_t* sel, unsigned long long* selq, ScanShared& sh,
+// radix threshold searches.  Same rules as select_small.
+static __device__ __noinline__ void select_and_draw(const SelectIn in, uint64_t* sel, unsigned long long* selq, ScanShared& sh,
                                              const RowOut o) {
     const int tid = threadIdx.x;
     const int n = in.n;
@@ -182,7 +182,6 @@ static __device__ __noinline__ bool select_and_draw(const SelectIn in, uint64_t*
         const uint64_t S = block_sum_u64(part, sh.red64);
         uint64_t Tp = __double2ull_rz(__dmul_rn((double)in.top_p, __ull2double_rn(in.S_ext ? in.S_ext : S)));
         if (Tp < 1) Tp = 1;
-        if (in.S_ext && !in.complete && S < Tp) return false;
         if (S >= Tp) {
             // dead entries take part with weight 0 (their keys are unique small numbers)
             const uint64_t C = block_radix_search<true, 56, false>(
@@ -197,7 +196,7 @@ static __device__ __noinline__ bool select_and_draw(const SelectIn in, uint64_t*
     const uint64_t S = block_sum_u64(part, sh.red64);
     if (S == 0) {
         row_fail(o, BORN_ROW_ALL_MASKED);
-        return true;
+        return;
     }
     uint64_t t = __double2ull_rz(__dmul_rn((double)in.u, __ull2double_rn(S)));
     if (t > S - 1) t = S - 1;
@@ -228,29 +227,18 @@ static __device__ __noinline__ bool select_and_draw(const SelectIn in, uint64_t*
         const uint64_t tot = block_sum_u64((uint64_t)alive, sh.red64);
         if (tid == 0 && o.kept_count) o.kept_count[o.row] = (int)tot;
     }
-    return true;
 }
 
-// Block-wide reductions of the compute threads (results to every thread).
-__device__ __forceinline__ float block_max_nan(float v, float* buf) {
-    v = warp_max_nan(v);
+// Block-wide reductions (results to every thread).
+__device__ __forceinline__ float block_max(float v, float* buf) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, d));
     cta_sync();
     if ((threadIdx.x & 31) == 0) buf[threadIdx.x >> 5] = v;
     cta_sync();
     float r = buf[0];
 #pragma unroll
-    for (int w = 1; w < kScanWarps; ++w) r = max_nan(r, buf[w]);
-    return r;
-}
-__device__ __forceinline__ float block_sum_f32(float v, float* buf) {
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-    cta_sync();
-    if ((threadIdx.x & 31) == 0) buf[threadIdx.x >> 5] = v;
-    cta_sync();
-    float r = 0.0f;
-#pragma unroll
-    for (int w = 0; w < kScanWarps; ++w) r += buf[w];
+    for (int w = 1; w < kScanWarps; ++w) r = fmaxf(r, buf[w]);
     return r;
 }
 
@@ -298,8 +286,8 @@ __device__ __forceinline__ float token_logit(const ScanArgs& A, const born_row_p
 // picks the block (ascending order, shares S_c), then the token inside it by the block's own
 // masses: t'' = min(floor((t - before) * M_c / S_c), M_c - 1) in float64.
 template <typename T>
-__device__ __forceinline__ void draw_whole_row(const ScanArgs& A, ScanShared& sh, uint8_t* scratch, const RowOut& o,
-                                               const born_row_params& rp, int b, int g, int row, float m, float inv_T,
+__device__ __forceinline__ void draw_whole_row(const ScanArgs& A, ScanShared& sh, const RowOut& o, const born_row_params& rp,
+                                               int b, int g, int row, float m, float inv_T,
                                                unsigned long long S, float u) {
     const int tid = threadIdx.x;
     const MassBlock* blocks = A.blocks + (int64_t)row * A.nblk;
@@ -386,178 +374,368 @@ __device__ __forceinline__ void draw_whole_row(const ScanArgs& A, ScanShared& sh
             o.prob[o.row] = __double2float_rn(p);
         }
     }
-    (void)scratch;
 }
 
-template <typename T>
-__device__ __noinline__ void fallback_row(const ScanArgs& A, ScanShared& sh, uint8_t* smem, int row);
-
-// Exactly the k best of a virtual row, in rank order, into its packed record.
-__device__ __forceinline__ void write_packed(const ScanArgs& A, ScanShared& sh, uint64_t* sel, unsigned long long* tmp_mem, int n, int k, int b, int g,
-                                             float m, float lse_s, float bound, bool exact) {
-    const int tid = threadIdx.x;
-    uint8_t* rec = A.packed + (int64_t)g * A.packed_seg_stride + (int64_t)b * A.packed_row_stride;
-    uint64_t* ent = reinterpret_cast<uint64_t*>(rec + kRecordHdrBytes);
-    int nk = 0;
-    if (exact && n > 0) {
-        if (n > kThreads) {
-            // cut to the k best first (k <= kThreads here), survivors to the front
-            const uint64_t Tk = block_radix_search<true, 56, true>(
-                n, (unsigned long long)(min(k, n) - 1), [&](int i) { return sel[i]; }, [&](int) { return 1ull; }, sh.sc);
-            uint64_t* tmp = reinterpret_cast<uint64_t*>(tmp_mem);  // the mass array is idle here
-            if (tid == 0) sh.nl = 0;
-            cta_sync();
-            for (int i = tid; i < n; i += kThreads)
-                if (sel[i] >= Tk) tmp[smem_atom_add(&sh.nl, 1u)] = sel[i];
-            cta_sync();
-            n = sh.nl;
-            for (int i = tid; i < n; i += kThreads) sel[i] = tmp[i];
-            cta_sync();
-        }
-        const uint64_t ck = tid < n ? sel[tid] : 0ull;
-        int rank = 0;
-        for (int j = 0; j < n; ++j) rank += (sel[j] > ck) ? 1 : 0;
-        nk = min(n, k);
-        if (tid < n && rank < nk) ent[rank] = ck;
+// Mass bins: a token z (scaled distance below the maximum x = (m - z) * inv_T) falls into bin
+// floor(32 x); masses are summed per bin as three 14-bit limbs in 32-bit words (32-bit shared-memory
+// atomics run at two cycles per warp here, 64-bit ones are compare-and-swap loops), which holds the
+// exact sum of up to 2^18 tokens.
+constexpr float kBinScale = 32.0f;
+__device__ __forceinline__ int nucleus_bin(float z, float m, float inv_T) {
+    return (int)fminf(__fmul_rn(__fmul_rn(__fsub_rn(m, z), inv_T), kBinScale), (float)(kBins - 1));
+}
+__device__ __forceinline__ void bin_mass(uint32_t* limb, int bin, uint64_t q) {
+    if (q == 0) return;
+    smem_red_add(&limb[bin], (uint32_t)q & 0x3FFFu);
+    smem_red_add(&limb[kBins + bin], (uint32_t)(q >> 14) & 0x3FFFu);
+    if (q >> 28) smem_red_add(&limb[2 * kBins + bin], (uint32_t)(q >> 28));
+}
+__device__ __forceinline__ uint64_t bin_total(const uint32_t* limb, int bin) {
+    return (uint64_t)limb[bin] + ((uint64_t)limb[kBins + bin] << 14) + ((uint64_t)limb[2 * kBins + bin] << 28);
+}
+// First bin at which the running total of `total_of(bin)` exceeds `target`, the total ahead of it in
+// `before`; -1 when the whole total does not.  All threads get the same answer.  (The caller's last
+// barrier covers the bins.)
+template <typename F>
+__device__ __forceinline__ int find_bin(F total_of, unsigned long long target, unsigned long long& before, ScanShared& sh) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int PER = kBins / kThreads;
+    uint64_t w[PER], loc = 0;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) { w[j] = total_of(PER * tid + j); loc += w[j]; }
+    uint64_t incl = loc;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint64_t up = shfl_up_u64(incl, d);
+        if (lane >= d) incl += up;
     }
-    if (tid == 0) {
-        PackedHdr h;
-        h.m = m; h.lse_s = lse_s; h.count = (uint32_t)nk;
-        h.flags = (exact ? 0u : 2u) | ((n > k) ? 1u : 0u);
-        h.bound = bound;
-        h.pad[0] = h.pad[1] = h.pad[2] = 0;
-        memcpy(rec, &h, sizeof h);
+    if (lane == 31) sh.red64[warp] = incl;
+    if (tid == 0) sh.found = -1;
+    cta_sync();
+    for (int i = 0; i < warp; ++i) incl += sh.red64[i];
+    if (incl > target && incl - loc <= target) {
+        uint64_t acc = incl - loc;
+        int j = 0;
+        for (; j < PER - 1 && acc + w[j] <= target; ++j) acc += w[j];
+        sh.found = PER * tid + j;
+        sh.before = acc;
     }
+    cta_sync();
+    before = sh.before;
+    return sh.found;
 }
 
-// Where a finished row's statistics and candidates come from: the segment records in scratch
-// (a row streamed by several CTAs), or -- when one CTA streamed the whole row -- that CTA's
-// own shared memory, without a round trip through L2.
+// A completed row: where its statistics, group keys and history values are.
 struct RowSrc {
-    bool direct;
-    float m, ls, taux, bk;       // direct: the row's maximum, log-sum-exp sum, exclusion level, lane-maxima bound
-    const uint64_t* wbuf;        // direct: the warps' candidate buffers (kScanWarps x kWarpCand raw entries)
-    const uint32_t* wcount;
+    int row, b, g;               // virtual row; caller row and vocabulary segment
+    bool direct;                 // one CTA streamed the whole row: statistics and history list in its shared memory
+    float m, ls;                 // direct: the row's maximum and log-sum-exp sum
+    const uint16_t* gkeys;       // group keys of the row
+    int hist_n;                  // direct: entries of the history list
     int c_first, nseg;           // records: CTAs that hold a segment of the row
-    int b, g;                    // the row: caller row and vocabulary segment
     float u;                     // the caller row's uniform, fetched while the row was streamed
     born_row_params rp;
     RowPlan plan;
 };
 
 // Hands row `row` to the exact search that its CTA runs once the ring is idle.  The reason goes in
-// the upper byte.  A CTA that streams exactly one row keeps the word in shared memory (and spares
-// every CTA a round trip to global memory at its end).
-template <bool kOneRow>
+// the upper byte.
 __device__ __forceinline__ void defer_row(const ScanArgs& A, ScanShared& sh, int row, uint32_t why) {
     const uint32_t word = (why << 24) | (blockIdx.x + 1u);
-    if constexpr (kOneRow) sh.defer = word;
-    else A.deferred[row] = word;
+    sh.defer = word;
+    if (A.slices == 0) A.deferred[row] = word;
 }
 
-// A row is complete: merge its statistics, select, draw.
-// kOneRow: the instantiation only ever finishes rows straight from the shared memory of the CTA
-// that streamed them, in sampling mode -- the record path and the k-best mode are left out of it.
-template <typename T, int kRoute, bool kOneRow>
-__device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, uint64_t* sel, unsigned long long* selq, int row,
-                                           const RowSrc& src) {
-    const int tid = threadIdx.x;
-    const bool direct = kOneRow || src.direct;
-    const bool local_mode = !kOneRow && A.mode == kScanLocal;
-    const int nseg = src.nseg, c_first = src.c_first;
-    const int b = src.b, g = src.g;
-    const born_row_params& rp = src.rp;
-    const RowPlan& pl = src.plan;
-    auto rec_of = [&](int s) { return A.records + (int64_t)(row + c_first + s) * A.rec_stride; };
+// The k-th largest of the row's group keys, from above, as far as the bins resolve it: a key that at
+// least k groups reach (so that at least k tokens do), and not many more.  Groups below the smallest
+// of the threads' own maxima cannot matter (at least as many groups reach that as there are threads;
+// for small k, quartets of threads), so the bins only span what is left.
+// All threads get the same answer; kDeadKey16 + 1 when fewer than k groups hold anything.
+__device__ __forceinline__ uint32_t kth_group_key(const uint16_t* keys, int ngrp, int k, uint32_t keym, uint32_t* bins, ScanShared& sh) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int kReg = 16;  // keys a thread keeps in registers: 4096 groups
+    uint32_t kk[kReg];
+    uint32_t mx = 0;
+#pragma unroll
+    for (int i = 0; i < kReg; ++i) {
+        const int g = tid + i * kThreads;
+        kk[i] = g < ngrp ? (uint32_t)keys[g] : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < kReg; ++i) mx = max(mx, kk[i]);
+    for (int g = tid + kReg * kThreads; g < ngrp; g += kThreads) mx = max(mx, (uint32_t)keys[g]);
+    if (k <= kThreads / 4) {
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    }
+    uint32_t lo = __reduce_min_sync(0xffffffffu, mx);
+    if (lane == 0) sh.redu[warp] = lo;
+    reinterpret_cast<uint4*>(bins)[tid] = make_uint4(0u, 0u, 0u, 0u);
+    cta_sync();
+#pragma unroll
+    for (int w = 0; w < kScanWarps; ++w) lo = min(lo, sh.redu[w]);
+    if (k > kThreads) lo = 0;
+    lo = max(lo, kDeadKey16 + 1u);
+    int s = 0;
+    while (keym >= lo && ((keym - lo) >> s) >= (uint32_t)kBins) ++s;
+#pragma unroll
+    for (int i = 0; i < kReg; ++i)
+        if (kk[i] >= lo) smem_red_add(&bins[(keym - kk[i]) >> s], 1u);
+    for (int g = tid + kReg * kThreads; g < ngrp; g += kThreads) {
+        const uint32_t key = keys[g];
+        if (key >= lo) smem_red_add(&bins[(keym - key) >> s], 1u);
+    }
+    cta_sync();
+    const uint4 c = reinterpret_cast<const uint4*>(bins)[tid];
+    uint32_t incl = c.x + c.y + c.z + c.w;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += up;
+    }
+    if (lane == 31) sh.redu[warp] = incl;
+    if (tid == 0) sh.found = -1;
+    cta_sync();
+    uint32_t off = 0;
+#pragma unroll
+    for (int w = 0; w < kScanWarps; ++w) off += w < warp ? sh.redu[w] : 0u;
+    const uint32_t before = off + incl - (c.x + c.y + c.z + c.w);
+    if (before < (uint32_t)k && off + incl >= (uint32_t)k) {
+        int j = 3;
+        if (before + c.x >= (uint32_t)k) j = 0;
+        else if (before + c.x + c.y >= (uint32_t)k) j = 1;
+        else if (before + c.x + c.y + c.z >= (uint32_t)k) j = 2;
+        sh.found = 4 * tid + j;
+    }
+    cta_sync();
+    const int b = sh.found;
+    if (b < 0) return kDeadKey16 + 1u;
+    const uint32_t span = ((uint32_t)(b + 1) << s) - 1u;  // (the lowest key of bin b)
+    return max(keym > span ? keym - span : 0u, lo);
+}
 
-    // statistics: row maximum, exclusion level, best lane-maxima bound, log-sum-exp sum
-    float m = src.m, taux = src.taux, bk = src.bk, ls = src.ls;
-    const bool cached = nseg <= kHdrCache;
-    if (!direct) {
-        m = -INFINITY; taux = -INFINITY; bk = -INFINITY; ls = 0.0f;
-        if (cached) {  // the headers are fetched once (one round trip to L2) and shared
-            cta_sync();
-            if (tid < nseg) {
-                const uint8_t* rec = rec_of(tid);
-                const float4 h = __ldcg(reinterpret_cast<const float4*>(rec));
-                sh.hdr[tid] = h;
-                sh.hdr_cnt[tid] = __ldcg(reinterpret_cast<const uint32_t*>(rec) + 4);
-            }
-            cta_sync();
-            for (int s = 0; s < nseg; ++s) {
-                const float4 h = sh.hdr[s];
-                m = max_nan(m, h.x);
-                taux = fmaxf(taux, h.z);
-                bk = fmaxf(bk, h.w);
-            }
-            if (!(RouteOf<kRoute>::mass && pl.need_mass))
-                for (int s = 0; s < nseg; ++s) {
-                    const float4 h = sh.hdr[s];
-                    if (h.y > 0.0f) ls += h.y * ex2_approx(__fmul_rn(h.x - m, pl.c2));
+// Raw logit of token `tok` of the row at `base` (no mask, no penalties).
+template <typename T>
+__device__ __forceinline__ float raw_logit(const uint8_t* base, int tok) {
+    if constexpr (sizeof(T) == 4) return __ldg(reinterpret_cast<const float*>(base) + tok);
+    else return bf16_bits_to_f32(__ldg(reinterpret_cast<const uint16_t*>(base) + tok));
+}
+
+// Every group of the row whose key reaches `tk`, read again: f(tok, z) with eight groups at a time, a
+// lane per token (z = -inf where there is none, or the mask hides it; no penalties).  A warp lists
+// the groups it finds among its share of the keys first, so that the re-reads leave eight at a time.
+template <typename T, typename F>
+__device__ __forceinline__ void for_groups(const ScanArgs& A, const uint16_t* keys, int b, int g, uint32_t tk, uint32_t* wl, F f) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ngrp = (A.V + kGrpTok - 1) / kGrpTok;
+    const uint8_t* base = reinterpret_cast<const uint8_t*>(A.logits) + ((int64_t)b * A.row_stride + (int64_t)g * A.V) * (int64_t)sizeof(T);
+    const uint32_t* mrow = A.mask ? A.mask + (int64_t)b * A.mask_stride : nullptr;
+    uint32_t* list = wl + warp * kGrpList;
+    int n = 0;
+    auto flush = [&]() {
+        __syncwarp();
+        for (int i = 0; i < n; i += 8) {
+            int tok[8];
+            float z[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) tok[e] = i + e < n ? (int)list[i + e] * kGrpTok + lane : A.V;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) z[e] = tok[e] < A.V ? raw_logit<T>(base, tok[e]) : -INFINITY;
+            if (mrow) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const int64_t bi = (int64_t)g * A.V + tok[e];
+                    if (tok[e] < A.V && !((__ldg(mrow + (bi >> 5)) >> (bi & 31)) & 1u)) z[e] = -INFINITY;
                 }
-        } else {
-            for (int s = tid; s < nseg; s += kThreads) {
-                const float4 h = __ldcg(reinterpret_cast<const float4*>(rec_of(s)));
-                m = max_nan(m, h.x);
-                taux = fmaxf(taux, h.z);
-                bk = fmaxf(bk, h.w);
             }
-            m = block_max_nan(m, sh.redf);
-            taux = block_max_nan(taux, sh.redf2);
-            bk = block_max_nan(bk, sh.redf3);
-            if (!(RouteOf<kRoute>::mass && pl.need_mass)) {
-                for (int s = tid; s < nseg; s += kThreads) {
-                    const float4 h = __ldcg(reinterpret_cast<const float4*>(rec_of(s)));
-                    if (h.y > 0.0f) ls += h.y * ex2_approx(__fmul_rn(h.x - m, pl.c2));
-                }
-                ls = block_sum_f32(ls, sh.redf);
+            f(tok, z);
+        }
+        __syncwarp();
+        n = 0;
+    };
+    for (int base_g = warp * 32; base_g < ngrp; base_g += 4 * kThreads) {
+        uint32_t key[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int gi = base_g + e * kThreads + lane;
+            key[e] = gi < ngrp ? (keys ? (uint32_t)keys[gi] : 0xFFFFu) : 0u;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const bool hit = key[e] >= tk;
+            const uint32_t hb = __ballot_sync(0xffffffffu, hit);
+            if (hit) list[n + __popc(hb & ((1u << lane) - 1u))] = (uint32_t)(base_g + e * kThreads + lane);
+            n += __popc(hb);
+        }
+        if (n > kGrpList - 128) flush();
+    }
+    if (n) flush();
+}
+
+// The row's history values: f(token of the virtual row, penalised value) for every entry, dealt over
+// the threads.
+template <typename F>
+__device__ __forceinline__ void for_history(const ScanArgs& A, const uint8_t* smem, const RowSrc& src, F f) {
+    if (src.direct) {
+        const unsigned long long* list = reinterpret_cast<const unsigned long long*>(smem + A.L.list);
+        for (int i = threadIdx.x; i < src.hist_n; i += kThreads) {
+            const unsigned long long e = list[i];
+            f((int)(uint32_t)e, __uint_as_float((uint32_t)(e >> 32)));
+        }
+    } else {
+        for (int s = 0; s < src.nseg; ++s) {
+            const uint8_t* rec = seg_record(A, src.row, src.c_first + s);
+            const int n = (int)__ldcg(reinterpret_cast<const uint32_t*>(rec) + 2);
+            const unsigned long long* ent = reinterpret_cast<const unsigned long long*>(rec + kRecordHdrBytes);
+            for (int i = threadIdx.x; i < n; i += kThreads) {
+                const unsigned long long e = __ldcg(ent + i);
+                f((int)(uint32_t)e, __uint_as_float((uint32_t)(e >> 32)));
             }
         }
     }
-    auto count_of = [&](int s) { return cached ? (int)sh.hdr_cnt[s] : (int)__ldcg(reinterpret_cast<const uint32_t*>(rec_of(s)) + 4); };
-    // every raw entry (value bits << 32 | token id) of the row, dealt over the threads
-    auto for_entries = [&](auto f) {
-        if (direct) {
-            for (int idx = tid; idx < kScanWarps * kWarpCand; idx += kThreads) {
-                const int w = idx / kWarpCand, i = idx - w * kWarpCand;
-                if (i < (int)min(src.wcount[w], (uint32_t)kWarpCand)) f(src.wbuf[idx]);
-            }
-        } else {
-            for (int s = 0; s < nseg; ++s) {
-                const int cnt = count_of(s);
-                const unsigned long long* ent = reinterpret_cast<const unsigned long long*>(rec_of(s) + kRecordHdrBytes);
-                for (int i = tid; i < cnt; i += kThreads) f(__ldcg(ent + i));
-            }
+}
+
+// Every token of the row at or above tau into sel (rank keys); returns their number, which may exceed
+// kSelCap (what does not fit is dropped: the caller looks at the number).  sh.nl is zero on entry.
+// A history token's raw value is struck out (its key keeps the index only, so that keys stay
+// unique) and its penalised value added.
+template <typename T, bool kHist>
+__device__ __forceinline__ int gather_row(const ScanArgs& A, ScanShared& sh, const uint8_t* smem, const RowSrc& src, float tau, uint64_t* sel,
+                                          uint32_t* wl) {
+    const int lane = threadIdx.x & 31;
+    const float tf = fmaxf(tau, -FLT_MAX);
+    const int id0 = A.idx_base + src.g * A.V;
+    for_groups<T>(A, src.gkeys, src.b, src.g, zkey(tf) >> 16, wl, [&](const int (&tok)[8], const float (&z)[8]) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const bool hit = z[e] >= tf;
+            const uint32_t hb = __ballot_sync(0xffffffffu, hit);
+            if (!hb) continue;
+            uint32_t pos = 0;
+            if (lane == 0) pos = smem_atom_add(&sh.nl, (uint32_t)__popc(hb));
+            pos = __shfl_sync(0xffffffffu, pos, 0) + __popc(hb & ((1u << lane) - 1u));
+            if (hit && pos < (uint32_t)kSelCap) sel[pos] = make_ck(z[e], id0 + tok[e]);
         }
-    };
+    });
+    cta_sync();
+    int n = sh.nl;
+    if constexpr (kHist) {
+        if (penalties_on(src.rp) && n <= kSelCap) {
+            for_history(A, smem, src, [&](int tok, float) {
+                const uint32_t low = kIdxMask - (uint32_t)(id0 + tok);
+                for (int i = 0; i < n; ++i)
+                    if ((uint32_t)(sel[i] & kIdxMask) == low) sel[i] = low;
+            });
+            cta_sync();
+            for_history(A, smem, src, [&](int tok, float zp) {
+                if (!(zp >= tf)) return;
+                const uint32_t pos = smem_atom_add(&sh.nl, 1u);
+                if (pos < (uint32_t)kSelCap) sel[pos] = make_ck(zp, id0 + tok);
+            });
+            cta_sync();
+            n = sh.nl;
+        }
+    }
+    return n;
+}
+
+// sel[0..n) cut to its k best (n > k), compacted through tmp; returns k.
+__device__ __forceinline__ int cut_to_k(uint64_t* sel, uint64_t* tmp, int n, int k, ScanShared& sh) {
+    const int tid = threadIdx.x;
+    const uint64_t Tk = block_radix_search<true, 56, true>(
+        n, (unsigned long long)(k - 1), [&](int i) { return sel[i]; }, [&](int) { return 1ull; }, sh.sc);
+    if (tid == 0) sh.nl = 0;
+    cta_sync();
+    for (int i = tid; i < n; i += kThreads)
+        if (sel[i] >= Tk) tmp[smem_atom_add(&sh.nl, 1u)] = sel[i];
+    cta_sync();
+    for (int i = tid; i < k; i += kThreads) sel[i] = tmp[i];
+    cta_sync();
+    return k;
+}
+
+// Exactly the k best of a virtual row (k <= kThreads), in rank order, into its packed record.
+__device__ __forceinline__ void write_packed(const ScanArgs& A, ScanShared& sh, uint64_t* sel, uint64_t* tmp, int n, int k, int b, int g,
+                                             float m, float lse_s) {
+    const int tid = threadIdx.x;
+    uint8_t* rec = A.packed + (int64_t)g * A.packed_seg_stride + (int64_t)b * A.packed_row_stride;
+    uint64_t* ent = reinterpret_cast<uint64_t*>(rec + kRecordHdrBytes);
+    if (n > kThreads) n = cut_to_k(sel, tmp, n, k, sh);
+    const uint64_t ck = tid < n ? sel[tid] : 0ull;
+    const int alive = cta_sync_count(tid < n && ck_alive(ck));
+    int rank = 0;
+    {
+        int j = 0;
+        for (; j + 8 <= n; j += 8) {
+            uint64_t v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = sel[j + i];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) rank += (v[i] > ck) ? 1 : 0;
+        }
+        for (; j < n; ++j) rank += (sel[j] > ck) ? 1 : 0;
+    }
+    const int nk = min(alive, k);
+    if (tid < n && rank < nk) ent[rank] = ck;
+    if (tid == 0) {
+        PackedHdr h;
+        h.m = m; h.lse_s = lse_s; h.count = (uint32_t)nk;
+        h.flags = alive > k ? 1u : 0u;
+        h.bound = -INFINITY;
+        h.pad[0] = h.pad[1] = h.pad[2] = 0;
+        memcpy(rec, &h, sizeof h);
+    }
+}
+
+template <typename T>
+__device__ __noinline__ void fallback_row(const ScanArgs& A, ScanShared& sh, uint8_t* smem, int row);
+
+// A row is complete: fold its statistics, select, draw.
+template <typename T, bool kHist, int kRoute>
+__device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, uint8_t* smem, const RowSrc& src) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int row = src.row, b = src.b, g = src.g;
+    const born_row_params& rp = src.rp;
+    const RowPlan& pl = src.plan;
+    const bool mass = RouteOf<kRoute>::mass && (!RouteOf<kRoute>::cand || pl.need_mass);
+    uint64_t* sel = reinterpret_cast<uint64_t*>(smem + A.L.work);
+    unsigned long long* selq = reinterpret_cast<unsigned long long*>(sel + kSelCap);
+    uint32_t* wl = reinterpret_cast<uint32_t*>(selq + kSelCap);
+    const int ngrp = (A.V + kGrpTok - 1) / kGrpTok;
+
+    float m = src.m, ls = src.ls;
+    if (!src.direct) {  // every warp folds the segments' headers for itself
+        m = -INFINITY;
+        for (int s = lane; s < src.nseg; s += 32) m = max_nan(m, __ldcg(reinterpret_cast<const float*>(seg_record(A, row, src.c_first + s))));
+        m = warp_max_nan(m);
+        ls = 0.0f;
+        if (!mass) {
+            for (int s = lane; s < src.nseg; s += 32) {
+                const float2 h = __ldcg(reinterpret_cast<const float2*>(seg_record(A, row, src.c_first + s)));
+                if (h.y > 0.0f) ls += h.y * ex2_approx(__fmul_rn(h.x - m, pl.c2));
+            }
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, d);
+        }
+    }
     int status = BORN_ROW_OK;
     if (m != m) status = BORN_ROW_NAN;
     else if (m == INFINITY) status = BORN_ROW_POS_INF;
     else if (m == -INFINITY) status = BORN_ROW_ALL_MASKED;
+    const uint32_t keym = zkey(m) >> 16;
 
-    if (local_mode) {
+    if (A.mode == kScanLocal) {
         // ---- the k best of the virtual row, in rank order
         int n = 0;
         if (status == BORN_ROW_OK) {
-            if (tid == 0) sh.nl = 0;
-            cta_sync();
-            for_entries([&](unsigned long long e) {
-                const float z = __uint_as_float((uint32_t)(e >> 32));
-                if (z >= bk && z >= taux) {
-                    const int pos = (int)smem_atom_add(&sh.nl, 1u);
-                    if (pos < kSelCap) sel[pos] = make_ck(z, (int)(uint32_t)e);
-                }
-            });
-            cta_sync();
-            n = sh.nl;
-            // complete above max(bk, taux); the k best are inside iff there are k of them (or nothing was excluded)
-            if (n > kSelCap || (taux > bk && n < pl.k) || (RouteOf<kRoute>::lane && pl.no_bound)) {
-                // the exact search over the row writes the record instead
-                if (tid == 0) defer_row<kOneRow>(A, sh, row, 8u);
+            const uint32_t tk = kth_group_key(src.gkeys, ngrp, pl.k, keym, reinterpret_cast<uint32_t*>(selq), sh);
+            n = gather_row<T, kHist>(A, sh, smem, src, zkey_to_float(tk << 16), sel, wl);
+            if (n > kSelCap) {
+                if (tid == 0) defer_row(A, sh, row, 8u);
                 return;
             }
         }
-        write_packed(A, sh, sel, selq, n, pl.k, b, g, m, ls, bk, true);
+        write_packed(A, sh, sel, reinterpret_cast<uint64_t*>(selq), n, pl.k, b, g, m, ls);
         return;
     }
 
@@ -571,22 +749,91 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
         row_fail(o, status);
         return;
     }
-    if (!(RouteOf<kRoute>::mass && pl.need_mass) && A.out_lse && tid == 0) A.out_lse[b] = m * pl.inv_T + __log2f(ls) * 0.69314718f;
+    if (!mass && A.out_lse && tid == 0) A.out_lse[b] = m * pl.inv_T + __log2f(ls) * 0.69314718f;
 
-    if (pl.greedy) {
-        if (taux > m) {  // a token equal to the maximum may have been lost to a full buffer
-            if (tid == 0) defer_row<kOneRow>(A, sh, row, 1u);
+    unsigned long long S_tot = 0;
+    float tau = -INFINITY;
+    if (RouteOf<kRoute>::mass && mass) {
+        // row total from the mass blocks; log-sum-exp from it
+        const MassBlock* blocks = A.blocks + (int64_t)row * A.nblk;
+        unsigned long long part = 0;
+        int fin = 0;
+        for (int c = tid; c < A.nblk; c += kThreads) {
+            const MassBlock bkc = load_block(blocks + c);
+            part += block_share(bkc, m, pl.inv_T);
+            fin += (int)bkc.pad;
+        }
+        S_tot = block_sum_u64(part, sh.red64);
+        if (S_tot == 0) {
+            row_fail(o, BORN_ROW_ALL_MASKED);
             return;
         }
-        uint64_t best = 0;
-        for_entries([&](unsigned long long e) {
-            const float z = __uint_as_float((uint32_t)(e >> 32));
-            if (z >= m) best = max(best, make_ck(z, (int)(uint32_t)e));
+        if (A.out_lse && tid == 0)
+            A.out_lse[b] = (float)((double)m * (double)pl.inv_T + log(__ull2double_rn(S_tot) * (1.0 / 1099511627776.0)));
+        if (!pl.window) {
+            if (A.out_kept_count) {
+                const int nfin = (int)block_sum_u64((uint64_t)fin, sh.red64);
+                if (tid == 0) A.out_kept_count[b] = nfin;
+            }
+            if (A.out_kept_ids) {  // the kept set is the whole row: no list of a useful size exists
+                if (tid == 0) defer_row(A, sh, row, 2u);
+                return;
+            }
+            draw_whole_row<T>(A, sh, o, rp, b, g, row, m, pl.inv_T, S_tot, src.u);
+            return;
+        }
+        if (kHist && penalties_on(rp)) {  // (the bins below would have to look every token up in the history)
+            if (tid == 0) defer_row(A, sh, row, 7u);
+            return;
+        }
+        // Nucleus of the whole row.  Tokens lighter than (1 - P) * S / V weigh less than (1 - P) * S
+        // together, so none of them is in it; the exact masses of the others go into bins of 1/32 of
+        // a scaled logit, and the bin in which the nucleus ends is the last one that matters.
+        const float s_all = (float)S_tot * (1.0f / 1099511627776.0f);
+        const float cut = fmaxf(m + (__logf((1.0f - rp.top_p) * s_all / (float)A.V) - 0.05f) * rp.temperature, -FLT_MAX);
+        uint32_t* limb = reinterpret_cast<uint32_t*>(sel);  // [3][kBins]
+        for (int i = tid; i < 3 * kBins / 4; i += kThreads) reinterpret_cast<uint4*>(limb)[i] = make_uint4(0u, 0u, 0u, 0u);
+        cta_sync();
+        for_groups<T>(A, src.gkeys, b, g, zkey(cut) >> 16, wl, [&](const int (&)[8], const float (&z)[8]) {
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+                uint64_t q[2];
+                mass2_of(make_float2(z[e], z[e + 1]), m, pl.inv_T, q[0], q[1]);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (z[e + h] >= cut) bin_mass(limb, nucleus_bin(z[e + h], m, pl.inv_T), q[h]);
+            }
         });
+        cta_sync();
+        unsigned long long Tp = __double2ull_rz(__dmul_rn((double)rp.top_p, __ull2double_rn(S_tot)));
+        if (Tp < 1) Tp = 1;
+        unsigned long long before;
+        const int bin = find_bin([&](int i) { return bin_total(limb, i); }, Tp - 1, before, sh);
+        if (bin < 0) {  // (the share of what was left out is an estimate)
+            if (tid == 0) defer_row(A, sh, row, 7u);
+            return;
+        }
+        // (a shade below the bin's lower edge: more candidates than needed do no harm)
+        tau = fmaxf(cut, m - ((float)(bin + 1) * (1.0f / kBinScale) + 0.002f) * rp.temperature - fabsf(m) * 1e-6f);
+    } else {
+        if (pl.greedy) tau = m;
+        if (pl.minp) tau = m + pl.delta;
+        if (pl.k > 0) {
+            const uint32_t tk = kth_group_key(src.gkeys, ngrp, pl.k, keym, reinterpret_cast<uint32_t*>(selq), sh);
+            tau = fmaxf(tau, zkey_to_float(tk << 16));
+        }
+    }
+    int n = gather_row<T, kHist>(A, sh, smem, src, tau, sel, wl);
+    if (n > kSelCap) {
+        if (tid == 0) defer_row(A, sh, row, mass ? 7u : pl.k > 0 ? 5u : pl.greedy ? 1u : 6u);
+        return;
+    }
+    if (RouteOf<kRoute>::cand && pl.greedy) {
+        uint64_t best = 0;
+        for (int i = tid; i < n; i += kThreads) best = max(best, (uint64_t)sel[i]);
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) best = max(best, shfl_xor_u64(best, d));
-        cta_sync();
-        if ((tid & 31) == 0) sh.red64[tid >> 5] = best;
+        if (lane == 0) sh.red64[tid >> 5] = best;
         cta_sync();
         if (tid == 0) {
             for (int w = 1; w < kScanWarps; ++w) best = max(best, (uint64_t)sh.red64[w]);
@@ -599,144 +846,16 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
         }
         return;
     }
-
-    const float u = src.u;
-    unsigned long long S_tot = 0;
-    if ((RouteOf<kRoute>::mass && pl.need_mass)) {
-        // row total from the mass blocks; log-sum-exp from it
-        const MassBlock* blocks = A.blocks + (int64_t)row * A.nblk;
-        unsigned long long part = 0;
-        int fin = 0;
-        for (int c = tid; c < A.nblk; c += kThreads) {
-            const MassBlock bkc = load_block(blocks + c);
-            part += block_share(bkc, m, pl.inv_T);
-            fin += (int)bkc.pad;
-        }
-        S_tot = block_sum_u64(part, sh.red64);
-        const int nfin = (int)block_sum_u64((uint64_t)fin, sh.red64);
-        if (S_tot == 0) {
-            row_fail(o, BORN_ROW_ALL_MASKED);
-            return;
-        }
-        if (A.out_lse && tid == 0)
-            A.out_lse[b] = (float)((double)m * (double)pl.inv_T + log(__ull2double_rn(S_tot) * (1.0 / 1099511627776.0)));
-        if (!(RouteOf<kRoute>::mass && pl.window)) {
-            if (A.out_kept_count && tid == 0) A.out_kept_count[b] = nfin;
-            if (A.out_kept_ids) {  // the kept set is the whole row: no list of a useful size exists
-                if (tid == 0) defer_row<kOneRow>(A, sh, row, 2u);
-                return;
-            }
-            draw_whole_row<T>(A, sh, nullptr, o, rp, b, g, row, m, pl.inv_T, S_tot, u);
-            return;
-        }
-    }
-
-    // ---- candidates at or above the valid cut
-    float cut = -INFINITY;
-    if ((RouteOf<kRoute>::lane && pl.lane_bound)) cut = bk;
-    if (rp.min_p > 0.0f) cut = fmaxf(cut, m + pl.delta);
-    if ((RouteOf<kRoute>::mass && pl.window)) {
-        // tokens lighter than (1 - P) * S / V weigh less than (1 - P) * S together: outside the nucleus
-        const float s_all = (float)S_tot * (1.0f / 1099511627776.0f);
-        cut = m + (__logf((1.0f - rp.top_p) * s_all / (float)A.V) - 0.05f) * rp.temperature;
-    }
-    bool complete = !(taux > cut);
-    float lowest = complete ? cut : taux;  // below it the entries are not all there: not used
-    // (sh.nl is zero on entry: the caller's last barrier saw to it)
-    auto gather = [&](float low) {
-        if (direct) {
-            // a warp compacts its own buffer: one reservation per 32 entries
-            const int lane = tid & 31, w = tid >> 5;
-            const uint32_t cnt = min(src.wcount[w], (uint32_t)kWarpCand);
-            const uint64_t* buf = src.wbuf + w * kWarpCand;
-            for (uint32_t base = 0; base < cnt; base += 32) {
-                const uint32_t i = base + lane;
-                const uint64_t e = i < cnt ? buf[i] : 0ull;
-                const float z = __uint_as_float((uint32_t)(e >> 32));
-                const bool ok = i < cnt && z >= low;
-                const uint32_t okb = __ballot_sync(0xffffffffu, ok);
-                if (!okb) continue;
-                uint32_t pos0 = 0;
-                if (lane == 0) pos0 = smem_atom_add(&sh.nl, (uint32_t)__popc(okb));
-                pos0 = __shfl_sync(0xffffffffu, pos0, 0);
-                const uint32_t pos = pos0 + __popc(okb & ((1u << lane) - 1u));
-                if (ok && pos < (uint32_t)kSelCap) sel[pos] = make_ck(z, (int)(uint32_t)e);
-            }
-        } else {
-            for_entries([&](unsigned long long e) {
-                const float z = __uint_as_float((uint32_t)(e >> 32));
-                if (z >= low) {
-                    const int pos = (int)smem_atom_add(&sh.nl, 1u);
-                    if (pos < kSelCap) sel[pos] = make_ck(z, (int)(uint32_t)e);
-                }
-            });
-        }
-        cta_sync();
-        return (int)sh.nl;
-    };
-    int n = gather(lowest);
-    if (n > kSelCap && !(RouteOf<kRoute>::lane && pl.no_bound)) {
-        // More candidates than the selection takes (a wide nucleus window, many ties).  Use only
-        // the part above a higher level -- the lowest of a fixed ladder (in scaled-logit units
-        // below the row maximum) that leaves at most kSelCap entries; that part is complete, and
-        // the checks below decide whether the kept set lies inside it.
-        constexpr int NL = 8;
-        const float ladder[NL] = {8.0f, 6.5f, 5.0f, 4.0f, 3.0f, 2.0f, 1.0f, 0.5f};
-        if (tid < NL) sh.sc.c[tid] = 0;
-        cta_sync();
-        for_entries([&](unsigned long long e) {
-            const float z = __uint_as_float((uint32_t)(e >> 32));
-            if (!(z >= lowest)) return;
-            const float d = (m - z) * pl.inv_T;
-            int lvl = -1;  // narrowest level that still holds the entry
-#pragma unroll
-            for (int l = 0; l < NL; ++l)
-                if (d <= ladder[l]) lvl = l;
-            if (lvl >= 0) smem_red_add(&sh.sc.c[lvl], 1u);
-        });
-        cta_sync();
-        int pick = -1;
-        uint32_t cum = 0;
-        // entries inside level l = those whose narrowest level is >= l: cumulative from the narrow end
-        for (int l = NL - 1; l >= 0; --l) {
-            cum += sh.sc.c[l];
-            if (cum <= (uint32_t)kSelCap) pick = l;
-        }
-        cta_sync();
-        if (pick >= 0) {
-            const float low2 = m - ladder[pick] * rp.temperature;
-            if (low2 > lowest) {
-                lowest = low2;
-                complete = false;
-                if (tid == 0) sh.nl = 0;
-                cta_sync();
-                n = gather(lowest);
-            }
-        }
-    }
-    // why a row goes to the exact search (kept in the upper byte of its `deferred` word)
-    uint32_t why = 0;
-    if ((RouteOf<kRoute>::lane && pl.no_bound)) why = 4;
-    else if (n > kSelCap) why = 3;
-    else if (!complete) {
-        if (pl.k > 0) { if (n < pl.k) why = 5; }   // the k best are all at or above taux iff k tokens are
-        else if (!(RouteOf<kRoute>::mass && pl.window)) why = 6;              // min-p survivors may lie below taux
-    }
-    bool defer = why != 0;
-    if (!defer) {
-        SelectIn in;
-        in.n = n;
-        in.k = pl.k;
-        in.Qa = (rp.min_p > 0.0f) ? __double2ull_ru((double)rp.min_p * 1099511627776.0) : 0ull;
-        in.top_p = rp.top_p;
-        in.S_ext = (RouteOf<kRoute>::mass && pl.window) ? S_tot : 0ull;
-        in.complete = complete;
-        in.m_row = m; in.inv_T = pl.inv_T; in.u = u;
-        if (n <= kThreads) defer = !select_small(in, sel, selq, sh, o);
-        else defer = !select_and_draw(in, sel, selq, sh, o);
-        if (defer) why = 7;                        // the nucleus reaches below the candidates
-    }
-    if (defer && tid == 0) defer_row<kOneRow>(A, sh, row, why);
+    if (pl.k > 0 && pl.k <= kThreads && n > kThreads) n = cut_to_k(sel, reinterpret_cast<uint64_t*>(selq), n, pl.k, sh);
+    SelectIn in;
+    in.n = n;
+    in.k = pl.k;
+    in.Qa = pl.minp ? __double2ull_ru((double)rp.min_p * 1099511627776.0) : 0ull;
+    in.top_p = rp.top_p;
+    in.S_ext = mass ? S_tot : 0ull;
+    in.m_row = m; in.inv_T = pl.inv_T; in.u = src.u;
+    if (n <= kThreads) select_small(in, sel, selq, sh, o);
+    else select_and_draw(in, sel, selq, sh, o);
 }
 
 }  // namespace born

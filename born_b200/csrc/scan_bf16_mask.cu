@@ -1,0 +1,8 @@
+// scan_kernel for bf16 launches with grammar masks and no token history.
+#include <cstdint>
+#define SCAN_INST_T uint16_t
+#define SCAN_INST_MASK true
+#define SCAN_INST_HIST false
+#define SCAN_INST_ATTRS scan_attrs_bf16_mask
+#define SCAN_INST_LAUNCH scan_launch_bf16_mask
+#include "scan_inst.cuh"

@@ -1,0 +1,8 @@
+// scan_kernel for fp32 launches with grammar masks and no token history.
+#include <cstdint>
+#define SCAN_INST_T float
+#define SCAN_INST_MASK true
+#define SCAN_INST_HIST false
+#define SCAN_INST_ATTRS scan_attrs_f32_mask
+#define SCAN_INST_LAUNCH scan_launch_f32_mask
+#include "scan_inst.cuh"
