@@ -45,6 +45,7 @@ struct Handle {
     int max_batch = 0, max_vocab = 0, max_k = 0;
     int num_sms = 0;
     int max_grid = 0;              // CTAs of the streaming kernel (two per SM)
+    int max_clusters[kClusterMax + 1] = {0};  // clusters of 2 .. kClusterMax of them that the GPU holds at once
     int max_rows = 0;              // virtual rows (caller rows x vocabulary segments) a call may stream
     int rec_slots = 0;             // segment records there is room for
     uint8_t* records = nullptr;    // segment records (kSegRecordBytes each)
@@ -171,6 +172,14 @@ bool host_need_mass(const born_row_params& p) {
     return !greedy && p.top_k <= 0 && !(p.min_p > 0.0f);
 }
 
+cudaError_t cluster_limits(int (&n)[kClusterMax + 1]) {
+    for (int c = 2; c <= kClusterMax; ++c) {
+        const cudaError_t e = scan_max_clusters(c, &n[c]);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 // The dynamic shared-memory limit of every instantiation is raised once (at create / first static call).
 cudaError_t scan_attrs_all() {
     cudaError_t e;
@@ -230,6 +239,7 @@ int fill_scan(Handle* h, ScanArgs& A, int B, int G, int V, int dtype, const void
     if ((uintptr_t)logits % esz) return fail(h, BORN_ERR_INVALID_ARGUMENT, "logits pointer is not aligned to its element size");
     if (mask && (uintptr_t)mask % 4) return fail(h, BORN_ERR_INVALID_ARGUMENT, "mask pointer is not 4-byte aligned");
     A.B = B; A.G = G; A.V = V;
+    A.cluster = 0;
     A.nb = (V + kBlkTok - 1) / kBlkTok;
     A.logits = logits; A.row_stride = row_stride;
     A.mask = mask; A.mask_stride = mask_stride;
@@ -242,17 +252,29 @@ int fill_scan(Handle* h, ScanArgs& A, int B, int G, int V, int dtype, const void
         int64_t s = h->max_grid / rows;
         const int64_t most = (A.nb + kMinSliceBlocks - 1) / kMinSliceBlocks;
         if (s > most) s = most;
-        if (s > 1 && rows * s > h->rec_slots) s = h->rec_slots / rows;
+        // Up to eight slices exchange through a cluster's shared memory, which saves some 2.5 us of
+        // tickets and record reads; so do more, if a slice stays short enough for one CTA to stream in
+        // a few microseconds (64 blocks, 256 KB of fp32).  All clusters have to fit at once: a second
+        // wave costs more than longer slices.
+        if (s > 1 && (s <= kClusterMax || A.nb <= 64 * kClusterMax)) {
+            int c = s < kClusterMax ? (int)s : kClusterMax;
+            while (c > 1 && h->max_clusters[c] < rows) --c;
+            if (c > 1) {
+                s = c;
+                A.cluster = 1;
+            }
+        }
+        if (!A.cluster && s > 1 && rows * s > h->rec_slots) s = h->rec_slots / rows;
         A.slices = s > 1 ? (int)s : 1;
         *grid = (int)rows * A.slices;
     } else {
         A.slices = 0;
         *grid = h->max_grid;
     }
-    A.L = scan_smem_layout(esz, rows_aligned(G, V, dtype, logits, row_stride), mask != nullptr, hist_cap, A.slices > 0, A.slices > 1 ? 0 : A.nb * 32,
+    A.L = scan_smem_layout(esz, rows_aligned(G, V, dtype, logits, row_stride), mask != nullptr, hist_cap, A.slices > 0, A.slices > 1 && !A.cluster ? 0 : A.nb * 32,
                            kScanSmemTwo);
     if (A.L.total > kScanSmemMax) return fail(h, BORN_ERR_UNSUPPORTED, "shared memory layout of %d bytes", A.L.total);
-    if ((A.slices != 1 || A.nb * 32 > A.L.gkeys_cap) && rows * A.nb * 32 > h->gkeys_cap)
+    if (((A.slices != 1 && !A.cluster) || A.nb * 32 > A.L.gkeys_cap) && rows * A.nb * 32 > h->gkeys_cap)
         return fail(h, BORN_ERR_UNSUPPORTED, "batch x vocab exceeds the workspace");
     A.records = h->records;
     A.gkeys = h->gkeys;
@@ -358,6 +380,7 @@ int32_t born_sampler_create(int32_t device, int32_t max_batch, int32_t max_vocab
     if (rc == BORN_OK && cudaMemset(h->tickets, 0, sp.tickets) != cudaSuccess) rc = BORN_ERR_CUDA;
     if (rc == BORN_OK && cudaMemset(h->dev_error, 0, 32 * sizeof(int)) != cudaSuccess) rc = BORN_ERR_CUDA;
     if (rc == BORN_OK && scan_attrs_all() != cudaSuccess) rc = BORN_ERR_CUDA;
+    if (rc == BORN_OK && cluster_limits(h->max_clusters) != cudaSuccess) rc = BORN_ERR_CUDA;
     if (rc == BORN_OK && spec_attrs_all() != cudaSuccess) rc = BORN_ERR_CUDA;
     for (int i = 0; i < 4 && rc == BORN_OK; ++i)
         if (cudaEventCreate(&h->ev[i]) != cudaSuccess) rc = BORN_ERR_CUDA;
@@ -1194,7 +1217,7 @@ extern "C" int32_t born_sample_static(const born_sample_args* a, void* stream) {
             cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess)
             return fail(nullptr, BORN_ERR_CUDA, "cudaDeviceGetAttribute failed");
         if (major != 10) return fail(nullptr, BORN_ERR_NO_DEVICE, "device %d is not sm_100; this library is built for sm_100a only", dev);
-        if ((e = scan_attrs_all()) != cudaSuccess)
+        if ((e = scan_attrs_all()) != cudaSuccess || (e = cluster_limits(h->max_clusters)) != cudaSuccess)
             return fail(nullptr, BORN_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
         h->device = dev;
         h->is_static = true;

@@ -270,7 +270,7 @@ __device__ __noinline__ void fallback_row(const ScanArgs& A, ScanShared& sh, uin
     // re-uses their place).  bf16 rows with penalties have history tokens that are not in them.
     c.gkeys = nullptr;
     if (A.slices > 0 && (!pl.need_mass || pl.window) && !(sizeof(T) == 2 && c.hist))
-        c.gkeys = A.slices == 1 && c.nb * 32 <= A.L.gkeys_cap ? reinterpret_cast<const uint16_t*>(smem + A.L.gkeys) : A.gkeys + (int64_t)row * (c.nb * 32);
+        c.gkeys = (A.slices == 1 || A.cluster) && c.nb * 32 <= A.L.gkeys_cap ? reinterpret_cast<const uint16_t*>(smem + A.L.gkeys) : A.gkeys + (int64_t)row * (c.nb * 32);
 
     // row maximum (the row is known to be valid: only rows with a finite maximum get here)
     {

@@ -53,8 +53,9 @@ struct SelectIn {
 // number of larger keys (keys are unique: the token index is part of them); candidates and
 // masses are then re-written in rank order, and since a mass never grows along that order the
 // kept set of every filter is a prefix of it, which every thread finds by walking the sorted
-// masses itself.
-__device__ __forceinline__ void select_small(const SelectIn& in, uint64_t* sel, unsigned long long* selq, ScanShared& sh,
+// masses itself.  Returns false when the nucleus of S_ext is not inside the candidates (nothing is
+// written then); all threads get the same answer.
+__device__ __forceinline__ bool select_small(const SelectIn& in, uint64_t* sel, unsigned long long* selq, ScanShared& sh,
                                              const RowOut& o) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = in.n;
@@ -120,9 +121,10 @@ __device__ __forceinline__ void select_small(const SelectIn& in, uint64_t* sel, 
     cta_sync();
     const int R = sh.nw;
     const uint64_t S = sh.acc[0];
+    if (topp && in.S_ext && S < Tp) return false;  // (uniform)
     if (S == 0) {  // cannot happen while the row maximum is finite; never divide by it
         row_fail(o, BORN_ROW_ALL_MASKED);
-        return;
+        return true;
     }
     uint64_t t = __double2ull_rz(__dmul_rn((double)in.u, __ull2double_rn(S)));
     if (t > S - 1) t = S - 1;
@@ -146,11 +148,12 @@ __device__ __forceinline__ void select_small(const SelectIn& in, uint64_t* sel, 
         if (o.kept_ids && tid < o.kept_stride) o.kept_ids[(int64_t)o.row * o.kept_stride + tid] = ck_idx(c2);
     }
     if (o.kept_count && tid == 0) o.kept_count[o.row] = R;
+    return true;
 }
 
 // Selection and draw over kThreads < n <= kSelCap candidates: radix select, then mass-weighted
 // radix threshold searches.  Same rules as select_small.
-static __device__ __noinline__ void select_and_draw(const SelectIn in, uint64_t* sel, unsigned long long* selq, ScanShared& sh,
+static __device__ __noinline__ bool select_and_draw(const SelectIn in, uint64_t* sel, unsigned long long* selq, ScanShared& sh,
                                              const RowOut o) {
     const int tid = threadIdx.x;
     const int n = in.n;
@@ -182,6 +185,7 @@ static __device__ __noinline__ void select_and_draw(const SelectIn in, uint64_t*
         const uint64_t S = block_sum_u64(part, sh.red64);
         uint64_t Tp = __double2ull_rz(__dmul_rn((double)in.top_p, __ull2double_rn(in.S_ext ? in.S_ext : S)));
         if (Tp < 1) Tp = 1;
+        if (in.S_ext && S < Tp) return false;
         if (S >= Tp) {
             // dead entries take part with weight 0 (their keys are unique small numbers)
             const uint64_t C = block_radix_search<true, 56, false>(
@@ -196,7 +200,7 @@ static __device__ __noinline__ void select_and_draw(const SelectIn in, uint64_t*
     const uint64_t S = block_sum_u64(part, sh.red64);
     if (S == 0) {
         row_fail(o, BORN_ROW_ALL_MASKED);
-        return;
+        return true;
     }
     uint64_t t = __double2ull_rz(__dmul_rn((double)in.u, __ull2double_rn(S)));
     if (t > S - 1) t = S - 1;
@@ -227,6 +231,7 @@ static __device__ __noinline__ void select_and_draw(const SelectIn in, uint64_t*
         const uint64_t tot = block_sum_u64((uint64_t)alive, sh.red64);
         if (tid == 0 && o.kept_count) o.kept_count[o.row] = (int)tot;
     }
+    return true;
 }
 
 // Block-wide reductions (results to every thread).
@@ -431,7 +436,8 @@ struct RowSrc {
     bool direct;                 // one CTA streamed the whole row: statistics and history list in its shared memory
     float m, ls;                 // direct: the row's maximum and log-sum-exp sum
     const uint16_t* gkeys;       // group keys of the row
-    int hist_n;                  // direct: entries of the history list
+    int hist_n;                  // direct: entries of the history list ...
+    int remote_hist;             // ... and those that other CTAs of the cluster left at its end
     int c_first, nseg;           // records: CTAs that hold a segment of the row
     float u;                     // the caller row's uniform, fetched while the row was streamed
     born_row_params rp;
@@ -446,44 +452,53 @@ __device__ __forceinline__ void defer_row(const ScanArgs& A, ScanShared& sh, int
     if (A.slices == 0) A.deferred[row] = word;
 }
 
-// The k-th largest of the row's group keys, from above, as far as the bins resolve it: a key that at
-// least k groups reach (so that at least k tokens do), and not many more.  Groups below the smallest
-// of the threads' own maxima cannot matter (at least as many groups reach that as there are threads;
-// for small k, quartets of threads), so the bins only span what is left.
-// All threads get the same answer; kDeadKey16 + 1 when fewer than k groups hold anything.
-__device__ __forceinline__ uint32_t kth_group_key(const uint16_t* keys, int ngrp, int k, uint32_t keym, uint32_t* bins, ScanShared& sh) {
+// The k-th largest of n 16-bit keys (key_of(i), zero: none), from above, as far as the bins resolve
+// it: a key that at least k of them reach, and not many more.  Keys below the smallest of the threads'
+// own maxima cannot matter (at least as many reach that as there are threads; for small k, pairs or
+// quartets of threads), so the bins -- equal steps of the value below the maximum m -- only span what is
+// left.  All threads get the same answer; kDeadKey16 + 1 when fewer than k are alive.
+template <typename F>
+__device__ __forceinline__ uint32_t kth_key(F key_of, int n, int k, float m, uint32_t* bins, ScanShared& sh) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int kReg = 16;  // keys a thread keeps in registers: 4096 groups
+    constexpr int kReg = 16;  // keys a thread keeps in registers: 4096 in all
     uint32_t kk[kReg];
-    uint32_t mx = 0;
+    uint32_t mx = 0, mn = 0xFFFFu;
+    auto see = [&](uint32_t key) {
+        mx = max(mx, key);
+        mn = min(mn, key > kDeadKey16 ? key : 0xFFFFu);
+    };
 #pragma unroll
     for (int i = 0; i < kReg; ++i) {
         const int g = tid + i * kThreads;
-        kk[i] = g < ngrp ? (uint32_t)keys[g] : 0u;
+        kk[i] = g < n ? key_of(g) : 0u;
     }
 #pragma unroll
-    for (int i = 0; i < kReg; ++i) mx = max(mx, kk[i]);
-    for (int g = tid + kReg * kThreads; g < ngrp; g += kThreads) mx = max(mx, (uint32_t)keys[g]);
-    if (k <= kThreads / 4) {
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    }
-    uint32_t lo = __reduce_min_sync(0xffffffffu, mx);
-    if (lane == 0) sh.redu[warp] = lo;
+    for (int i = 0; i < kReg; ++i) see(kk[i]);
+    for (int g = tid + kReg * kThreads; g < n; g += kThreads) see(key_of(g));
+    if (k <= kThreads / 2) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    if (k <= kThreads / 4) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    const uint32_t lo_w = __reduce_min_sync(0xffffffffu, mx), mn_w = __reduce_min_sync(0xffffffffu, mn);
+    if (lane == 0) sh.redu[warp] = (lo_w << 16) | mn_w;
     reinterpret_cast<uint4*>(bins)[tid] = make_uint4(0u, 0u, 0u, 0u);
     cta_sync();
+    uint32_t lo = 0xFFFFu;
+    mn = 0xFFFFu;
 #pragma unroll
-    for (int w = 0; w < kScanWarps; ++w) lo = min(lo, sh.redu[w]);
-    if (k > kThreads) lo = 0;
-    lo = max(lo, kDeadKey16 + 1u);
-    int s = 0;
-    while (keym >= lo && ((keym - lo) >> s) >= (uint32_t)kBins) ++s;
+    for (int w = 0; w < kScanWarps; ++w) {
+        const uint32_t x = sh.redu[w];
+        lo = min(lo, x >> 16);
+        mn = min(mn, x & 0xFFFFu);
+    }
+    lo = max(k > kThreads ? 0u : lo, mn);
+    const float span = m - zkey_to_float(lo << 16);
+    const float scale = span > 0.0f ? (float)(kBins - 1) / span : 0.0f;
+    auto bin_of = [&](uint32_t key) { return (int)fminf(__fmul_rn(m - zkey_to_float(key << 16), scale), (float)(kBins - 1)); };
 #pragma unroll
     for (int i = 0; i < kReg; ++i)
-        if (kk[i] >= lo) smem_red_add(&bins[(keym - kk[i]) >> s], 1u);
-    for (int g = tid + kReg * kThreads; g < ngrp; g += kThreads) {
-        const uint32_t key = keys[g];
-        if (key >= lo) smem_red_add(&bins[(keym - key) >> s], 1u);
+        if (kk[i] >= lo) smem_red_add(&bins[bin_of(kk[i])], 1u);
+    for (int g = tid + kReg * kThreads; g < n; g += kThreads) {
+        const uint32_t key = key_of(g);
+        if (key >= lo) smem_red_add(&bins[bin_of(key)], 1u);
     }
     cta_sync();
     const uint4 c = reinterpret_cast<const uint4*>(bins)[tid];
@@ -510,8 +525,9 @@ __device__ __forceinline__ uint32_t kth_group_key(const uint16_t* keys, int ngrp
     cta_sync();
     const int b = sh.found;
     if (b < 0) return kDeadKey16 + 1u;
-    const uint32_t span = ((uint32_t)(b + 1) << s) - 1u;  // (the lowest key of bin b)
-    return max(keym > span ? keym - span : 0u, lo);
+    if (b == kBins - 1 || scale == 0.0f) return lo;
+    // the lowest key of bin b (a key lower: the bins' own rounding)
+    return max((zkey(m - __fdiv_rn((float)(b + 1), scale)) >> 16) - 1u, lo);
 }
 
 // Raw logit of token `tok` of the row at `base` (no mask, no penalties).
@@ -576,23 +592,45 @@ __device__ __forceinline__ void for_groups(const ScanArgs& A, const uint16_t* ke
 // the threads.
 template <typename F>
 __device__ __forceinline__ void for_history(const ScanArgs& A, const uint8_t* smem, const RowSrc& src, F f) {
+    auto one = [&](unsigned long long e) { f((int)(uint32_t)e, __uint_as_float((uint32_t)(e >> 32))); };
     if (src.direct) {
         const unsigned long long* list = reinterpret_cast<const unsigned long long*>(smem + A.L.list);
-        for (int i = threadIdx.x; i < src.hist_n; i += kThreads) {
-            const unsigned long long e = list[i];
-            f((int)(uint32_t)e, __uint_as_float((uint32_t)(e >> 32)));
-        }
-    } else {
-        for (int s = 0; s < src.nseg; ++s) {
-            const uint8_t* rec = seg_record(A, src.row, src.c_first + s);
-            const int n = (int)__ldcg(reinterpret_cast<const uint32_t*>(rec) + 2);
-            const unsigned long long* ent = reinterpret_cast<const unsigned long long*>(rec + kRecordHdrBytes);
-            for (int i = threadIdx.x; i < n; i += kThreads) {
-                const unsigned long long e = __ldcg(ent + i);
-                f((int)(uint32_t)e, __uint_as_float((uint32_t)(e >> 32)));
-            }
+        for (int i = threadIdx.x; i < src.hist_n; i += kThreads) one(list[i]);
+        for (int i = threadIdx.x; i < src.remote_hist; i += kThreads) one(list[A.L.list_cap - 1 - i]);
+        return;
+    }
+    const int lane = threadIdx.x & 31;
+    for (int s0 = 0; s0 < src.nseg; s0 += 32) {
+        uint32_t cnt = 0;
+        if (s0 + lane < src.nseg) cnt = __ldcg(reinterpret_cast<const uint32_t*>(seg_record(A, src.row, src.c_first + s0 + lane)) + 2);
+        for (int s = s0; s < min(src.nseg, s0 + 32); ++s) {
+            const int n = (int)__shfl_sync(0xffffffffu, cnt, s - s0);
+            const unsigned long long* ent = reinterpret_cast<const unsigned long long*>(seg_record(A, src.row, src.c_first + s) + kRecordHdrBytes);
+            for (int i = threadIdx.x; i < n; i += kThreads) one(__ldcg(ent + i));
         }
     }
+}
+// ... and an upper bound of how many there are.
+__device__ __forceinline__ int history_bound(const ScanArgs& A, const RowSrc& src) {
+    if (!penalties_on(src.rp)) return 0;
+    return src.direct ? src.hist_n + src.remote_hist : A.history_stride;
+}
+
+// The key that the k best tokens of the row reach.  From the group keys where there are enough groups
+// for their maxima to tell tokens apart; on shorter rows (some 40 k tokens) from the tokens
+// themselves, of which `extra` may not count (history tokens: their raw values).
+template <typename T>
+__device__ __forceinline__ uint32_t kth_token_key(const ScanArgs& A, const RowSrc& src, int k, int extra, float m, uint32_t* bins, ScanShared& sh) {
+    const int ngrp = (A.V + kGrpTok - 1) / kGrpTok;
+    if (4 * ngrp >= 5 * k) return kth_key([&](int i) { return (uint32_t)src.gkeys[i]; }, ngrp, k, m, bins, sh);
+    const uint8_t* base = reinterpret_cast<const uint8_t*>(A.logits) + ((int64_t)src.b * A.row_stride + (int64_t)src.g * A.V) * (int64_t)sizeof(T);
+    const uint32_t* mrow = A.mask ? A.mask + (int64_t)src.b * A.mask_stride : nullptr;
+    return kth_key([&](int i) {
+        const int64_t bi = (int64_t)src.g * A.V + i;
+        const float z = raw_logit<T>(base, i);
+        const bool hidden = (mrow && !((__ldg(mrow + (bi >> 5)) >> (bi & 31)) & 1u)) || z != z;
+        return hidden ? 0u : min(zkey(z), zkey(m)) >> 16;  // (a raw history value may lie above the maximum)
+    }, A.V, k + extra, m, bins, sh);
 }
 
 // Every token of the row at or above tau into sel (rank keys); returns their number, which may exceed
@@ -606,15 +644,21 @@ __device__ __forceinline__ int gather_row(const ScanArgs& A, ScanShared& sh, con
     const float tf = fmaxf(tau, -FLT_MAX);
     const int id0 = A.idx_base + src.g * A.V;
     for_groups<T>(A, src.gkeys, src.b, src.g, zkey(tf) >> 16, wl, [&](const int (&tok)[8], const float (&z)[8]) {
+        uint32_t hb[8], sum = 0;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            const bool hit = z[e] >= tf;
-            const uint32_t hb = __ballot_sync(0xffffffffu, hit);
-            if (!hb) continue;
-            uint32_t pos = 0;
-            if (lane == 0) pos = smem_atom_add(&sh.nl, (uint32_t)__popc(hb));
-            pos = __shfl_sync(0xffffffffu, pos, 0) + __popc(hb & ((1u << lane) - 1u));
-            if (hit && pos < (uint32_t)kSelCap) sel[pos] = make_ck(z[e], id0 + tok[e]);
+            hb[e] = __ballot_sync(0xffffffffu, z[e] >= tf);
+            sum += __popc(hb[e]);
+        }
+        if (sum == 0) return;
+        uint32_t pos = 0;
+        if (lane == 0) pos = smem_atom_add(&sh.nl, sum);
+        pos = __shfl_sync(0xffffffffu, pos, 0);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const uint32_t at = pos + __popc(hb[e] & ((1u << lane) - 1u));
+            if (z[e] >= tf && at < (uint32_t)kSelCap) sel[at] = make_ck(z[e], id0 + tok[e]);
+            pos += __popc(hb[e]);
         }
     });
     cta_sync();
@@ -722,13 +766,12 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
     if (m != m) status = BORN_ROW_NAN;
     else if (m == INFINITY) status = BORN_ROW_POS_INF;
     else if (m == -INFINITY) status = BORN_ROW_ALL_MASKED;
-    const uint32_t keym = zkey(m) >> 16;
 
     if (A.mode == kScanLocal) {
         // ---- the k best of the virtual row, in rank order
         int n = 0;
         if (status == BORN_ROW_OK) {
-            const uint32_t tk = kth_group_key(src.gkeys, ngrp, pl.k, keym, reinterpret_cast<uint32_t*>(selq), sh);
+            const uint32_t tk = kth_token_key<T>(A, src, pl.k, kHist ? history_bound(A, src) : 0, m, reinterpret_cast<uint32_t*>(selq), sh);
             n = gather_row<T, kHist>(A, sh, smem, src, zkey_to_float(tk << 16), sel, wl);
             if (n > kSelCap) {
                 if (tid == 0) defer_row(A, sh, row, 8u);
@@ -786,29 +829,49 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
             if (tid == 0) defer_row(A, sh, row, 7u);
             return;
         }
-        // Nucleus of the whole row.  Tokens lighter than (1 - P) * S / V weigh less than (1 - P) * S
-        // together, so none of them is in it; the exact masses of the others go into bins of 1/32 of
-        // a scaled logit, and the bin in which the nucleus ends is the last one that matters.
+        // Nucleus of the whole row: a value that the tokens of the nucleus all reach.  First from the
+        // group keys alone -- if the groups' best tokens, their values rounded down, already hold the
+        // nucleus' share above some value, so do all tokens above it.  Exact masses go into bins of
+        // 1/32 of a scaled logit; the bin in which the share is reached is the last that matters.
+        // Flat rows, where a group has more than one token that counts, take the tokens themselves:
+        // tokens lighter than (1 - P) * S / V weigh less than (1 - P) * S together, so none of those is
+        // in the nucleus, and the groups that reach beyond them are read again.
         const float s_all = (float)S_tot * (1.0f / 1099511627776.0f);
         const float cut = fmaxf(m + (__logf((1.0f - rp.top_p) * s_all / (float)A.V) - 0.05f) * rp.temperature, -FLT_MAX);
-        uint32_t* limb = reinterpret_cast<uint32_t*>(sel);  // [3][kBins]
-        for (int i = tid; i < 3 * kBins / 4; i += kThreads) reinterpret_cast<uint4*>(limb)[i] = make_uint4(0u, 0u, 0u, 0u);
-        cta_sync();
-        for_groups<T>(A, src.gkeys, b, g, zkey(cut) >> 16, wl, [&](const int (&)[8], const float (&z)[8]) {
-#pragma unroll
-            for (int e = 0; e < 8; e += 2) {
-                uint64_t q[2];
-                mass2_of(make_float2(z[e], z[e + 1]), m, pl.inv_T, q[0], q[1]);
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    if (z[e + h] >= cut) bin_mass(limb, nucleus_bin(z[e + h], m, pl.inv_T), q[h]);
-            }
-        });
-        cta_sync();
         unsigned long long Tp = __double2ull_rz(__dmul_rn((double)rp.top_p, __ull2double_rn(S_tot)));
         if (Tp < 1) Tp = 1;
+        uint32_t* limb = reinterpret_cast<uint32_t*>(sel);  // [3][kBins]
         unsigned long long before;
-        const int bin = find_bin([&](int i) { return bin_total(limb, i); }, Tp - 1, before, sh);
+        int bin = -1;
+        for (int level = 0; level < 2 && bin < 0; ++level) {
+            for (int i = tid; i < 3 * kBins / 4; i += kThreads) reinterpret_cast<uint4*>(limb)[i] = make_uint4(0u, 0u, 0u, 0u);
+            cta_sync();
+            if (level == 0) {
+                const uint32_t ck16 = zkey(cut) >> 16;
+                for (int i = tid; i < ngrp; i += 2 * kThreads) {
+                    const uint32_t k0 = src.gkeys[i], k1 = i + kThreads < ngrp ? (uint32_t)src.gkeys[i + kThreads] : 0u;
+                    const float z0 = zkey_to_float(k0 << 16), z1 = zkey_to_float(max(k1, 0x80u) << 16);
+                    uint64_t q0, q1;
+                    mass2_of(make_float2(z0, z1), m, pl.inv_T, q0, q1);
+                    if (k0 >= ck16) bin_mass(limb, nucleus_bin(z0, m, pl.inv_T), q0);
+                    if (k1 >= ck16) bin_mass(limb, nucleus_bin(z1, m, pl.inv_T), q1);
+                }
+            } else {
+                for_groups<T>(A, src.gkeys, b, g, zkey(cut) >> 16, wl, [&](const int (&)[8], const float (&z)[8]) {
+#pragma unroll
+                    for (int e = 0; e < 8; e += 2) {
+                        uint64_t q[2];
+                        mass2_of(make_float2(z[e], z[e + 1]), m, pl.inv_T, q[0], q[1]);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            if (z[e + h] >= cut) bin_mass(limb, nucleus_bin(z[e + h], m, pl.inv_T), q[h]);
+                    }
+                });
+            }
+            cta_sync();
+            bin = find_bin([&](int i) { return bin_total(limb, i); }, Tp - 1, before, sh);
+            cta_sync();
+        }
         if (bin < 0) {  // (the share of what was left out is an estimate)
             if (tid == 0) defer_row(A, sh, row, 7u);
             return;
@@ -819,7 +882,7 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
         if (pl.greedy) tau = m;
         if (pl.minp) tau = m + pl.delta;
         if (pl.k > 0) {
-            const uint32_t tk = kth_group_key(src.gkeys, ngrp, pl.k, keym, reinterpret_cast<uint32_t*>(selq), sh);
+            const uint32_t tk = kth_token_key<T>(A, src, pl.k, kHist ? history_bound(A, src) : 0, m, reinterpret_cast<uint32_t*>(selq), sh);
             tau = fmaxf(tau, zkey_to_float(tk << 16));
         }
     }
@@ -854,8 +917,8 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
     in.top_p = rp.top_p;
     in.S_ext = mass ? S_tot : 0ull;
     in.m_row = m; in.inv_T = pl.inv_T; in.u = src.u;
-    if (n <= kThreads) select_small(in, sel, selq, sh, o);
-    else select_and_draw(in, sel, selq, sh, o);
+    const bool inside = n <= kThreads ? select_small(in, sel, selq, sh, o) : select_and_draw(in, sel, selq, sh, o);
+    if (!inside && tid == 0) defer_row(A, sh, row, 7u);
 }
 
 }  // namespace born

@@ -7,8 +7,10 @@
 // every row is given `slices` CTAs of its own, each with one segment; beyond that the blocks of
 // all rows form one sequence that is cut into equal contiguous ranges, one per CTA, so that a CTA
 // may end in mid-row.  A row that one CTA streamed from first to last block is finished by it
-// at once; otherwise the segments leave records in scratch and the CTA that completes the row
-// (atomic ticket, no spinning) finishes it.
+// at once.  The slices of a row, up to eight, form a thread-block cluster: they write their keys,
+// history values and statistics straight into the first one's shared memory, which finishes the row
+// after one cluster barrier.  Otherwise (more slices, or ranges) the segments leave records in scratch
+// and the CTA that completes the row (atomic ticket, no spinning) finishes it.
 //
 // What a segment leaves behind is small and never overflows: its statistics, and one 16-bit key
 // per group of 32 tokens -- the upper half of the order-preserving key of the group's maximum.  The
@@ -28,6 +30,7 @@ constexpr int kScanStagesMax = 8;           // slots per warp ring, at most
 constexpr int kMassBlock = 512;             // tokens per mass block of the whole-vocabulary routes: half a warp's block
 constexpr int kSelCap = 1024;               // candidates the in-shared-memory selection handles
 constexpr int kHistBuckets = 128;           // the history list of a segment is grouped by block (or run of blocks)
+constexpr int kClusterMax = 8;              // slices of a row that exchange through distributed shared memory
 constexpr int kGrpList = 256;               // groups a warp lists before it reads them again
 constexpr int kBins = 1024;                 // bins of the finish's histograms
 constexpr uint32_t kDeadKey16 = 0x7Fu;      // group key of a group with nothing above -inf (-inf itself: 0x007FFFFF)
@@ -99,6 +102,7 @@ struct ScanArgs {
     int V;         // tokens per virtual row
     int nb;        // blocks per virtual row
     int slices;    // CTAs per virtual row; 0: contiguous ranges of blocks instead
+    int cluster;   // the slices of a row are a thread-block cluster
     int mode;      // kScanFull: sample; kScanLocal: leave the k best of every virtual row in `packed`
     int want_lse;
     int idx_base;  // added to the token ids written in kScanLocal mode
@@ -115,6 +119,19 @@ struct ScanArgs {
     long long debug_skip_blk;       // test hook: the bulk copy of this block is never issued (-1: none)
     ScanSmem L;
 };
+
+// ---- thread-block clusters ------------------------------------------------------------------
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Generic address of `p` (this CTA's shared memory) in CTA `rank` of the cluster.
+template <typename P>
+__device__ __forceinline__ P* cluster_map(P* p, uint32_t rank) {
+    unsigned long long r;
+    asm volatile("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(p), "r"(rank));
+    return reinterpret_cast<P*>(r);
+}
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- geometry -----------------------------------------------------------------------------
 struct RowGeom {
@@ -193,7 +210,9 @@ inline ScanSmem scan_smem_layout(int elem_bytes, bool aligned, bool has_mask, in
 struct ScanShared {
     unsigned long long bars[kScanStagesMax * kScanWarps];
     float wmax[kScanWarps], wsum[kScanWarps];
-    int fail;
+    float2 part[kClusterMax];       // cluster: (maximum, log-sum-exp sum) of every slice, in the first one
+    uint32_t remote_hist;           // cluster: history entries the other slices have left at the list's end
+    int remote_fail;                // cluster: a wait of another slice ran out
     uint32_t defer;                 // the CTA has handed a row to the exact search: its `deferred` word (0: none)
     int last;
     // finish / selection scratch

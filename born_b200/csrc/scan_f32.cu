@@ -5,4 +5,5 @@
 #define SCAN_INST_HIST false
 #define SCAN_INST_ATTRS scan_attrs_f32
 #define SCAN_INST_LAUNCH scan_launch_f32
+#define SCAN_INST_CLUSTERS scan_max_clusters
 #include "scan_inst.cuh"

@@ -19,14 +19,35 @@ namespace {
 template <bool kAligned, int R>
 constexpr auto kernel_of = scan_kernel<SCAN_INST_T, SCAN_INST_MASK, SCAN_INST_HIST, kAligned, R>;
 
+void scan_launch_config(const ScanArgs& A, int grid, cudaStream_t st, cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&at)[2]) {
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDim = dim3((unsigned)grid, 1, 1);
+    cfg.blockDim = dim3(kScanThreads, 1, 1);
+    cfg.dynamicSmemBytes = (size_t)A.L.total;
+    cfg.stream = st;
+    cfg.attrs = at;
+    int n = 0;
+    if (A.cluster) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = (unsigned)A.slices;
+        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = (unsigned)(n + 1);
+}
+
 template <bool kAligned, int R>
 cudaError_t attr_one() {
     return cudaFuncSetAttribute(kernel_of<kAligned, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmemMax);
 }
 template <bool kAligned, int R>
 cudaError_t launch_one(const ScanArgs& A, int grid, cudaStream_t st) {
-    kernel_of<kAligned, R><<<grid, kScanThreads, A.L.total, st>>>(A);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[2];
+    scan_launch_config(A, grid, st, cfg, at);
+    return cudaLaunchKernelEx(&cfg, kernel_of<kAligned, R>, A);
 }
 
 }  // namespace
@@ -40,6 +61,23 @@ cudaError_t SCAN_INST_ATTRS() {
     if ((e = attr_one<true, 2>()) != cudaSuccess) return e;
     return attr_one<false, 1>();
 }
+
+#ifdef SCAN_INST_CLUSTERS
+// Clusters of `size` CTAs that the current device holds at once (any instantiation: they share the
+// register and shared-memory budget of two CTAs per SM).
+cudaError_t SCAN_INST_CLUSTERS(int size, int* count) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[2];
+    ScanArgs A;
+    memset(&A, 0, sizeof A);
+    A.cluster = 1;
+    A.slices = size;
+    A.L.total = kScanSmemTwo;
+    scan_launch_config(A, size, nullptr, cfg, at);
+    cfg.numAttrs = 1;
+    return cudaOccupancyMaxActiveClusters(count, kernel_of<true, 1>, &cfg);
+}
+#endif
 
 cudaError_t SCAN_INST_LAUNCH(const ScanArgs& A, bool aligned, int route, int grid, cudaStream_t st) {
     if (!aligned) return route == 1 ? launch_one<false, 1>(A, grid, st) : cudaErrorInvalidValue;

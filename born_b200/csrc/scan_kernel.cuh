@@ -328,13 +328,24 @@ __global__ void __launch_bounds__(kScanThreads, 2) scan_kernel(const __grid_cons
         for (int s = 0; s < S; ++s) mbar_init(reinterpret_cast<uint64_t*>(&sh.bars[s * kScanWarps + warp]), 1);
         mbar_fence_init();
     }
-    if (tid == 0) { sh.fail = 0; sh.defer = 0; }
+    if (tid == 0) { sh.defer = 0; sh.remote_hist = 0; sh.remote_fail = 0; }
     __syncwarp();
+    // Everything above runs while the launch before this one may still be working (programmatic
+    // dependent launch); nothing below starts before its results are there.
+    grid_launch_dependents();
+    grid_dependency_wait();
+    if (A.cluster) cluster_arrive();  // (waited for before the first access to another CTA's shared memory)
     int ids[kHistPer];
     BlockCursor<T> ci;  // the copies' walk
     long long ti = t0 + warp;
     ci.start(A, ti < t1 ? ti : t0);
-    if constexpr (kHist) hist_ids(A, A.slices > 0 ? ci.q.b : (int)(t0 / nb) / A.G, ids);
+    // The first row's parameters, history ids and uniform go ahead of the bulk copies: behind them
+    // they would wait in the memory system's queues.
+    BlockCursor<T> c0;
+    c0.start(A, t0);
+    born_row_params rp = A.row_params ? A.row_params[c0.q.b] : A.params;
+    float u_row = (A.uniforms != nullptr && A.mode == kScanFull) ? __ldg(A.uniforms + c0.q.b) : 0.0f;
+    if constexpr (kHist) hist_ids(A, c0.q.b, ids);
     uint32_t si = 0;    // slot of the next copy
     auto issue = [&]() {
         if (lane == 0) issue_block<T, kMask, kAligned>(A, ci.q, ci.j, ti, slot0 + si * (kScanWarps * slot_bytes), bar0 + si * (kScanWarps * 8u));
@@ -354,22 +365,24 @@ __global__ void __launch_bounds__(kScanThreads, 2) scan_kernel(const __grid_cons
     bool first_seg = true;
     while (t < t1) {
         // ---- segment set-up (block-synchronous)
-        BlockCursor<T> c0;
-        c0.start(A, t);
+        if (!first_seg) {
+            c0.start(A, t);
+            rp = A.row_params ? A.row_params[c0.q.b] : A.params;
+            u_row = (A.uniforms != nullptr && A.mode == kScanFull) ? __ldg(A.uniforms + c0.q.b) : 0.0f;
+        }
         const int row = c0.row, j0 = c0.j;
         const RowGeom q = c0.q;
         const long long row_t0 = (long long)row * nb;
         const long long te = min(t1, row_t0 + nb);
         const bool whole = j0 == 0 && te == row_t0 + nb;
-        const born_row_params rp = A.row_params ? A.row_params[q.b] : A.params;
         const RowPlan pl = row_plan(rp);
         const bool mass = RouteOf<kRoute>::mass && (!RouteOf<kRoute>::cand || pl.need_mass);
         const bool want_lse = !mass && (A.out_lse != nullptr || A.want_lse);
-        // the row's uniform is wanted at the very end: fetch it now
-        const float u_row = (A.uniforms != nullptr && A.mode == kScanFull) ? __ldg(A.uniforms + q.b) : 0.0f;
-        // group keys: shared memory when this CTA finishes the row and there is room
-        const bool keys_smem = whole && nb * 32 <= A.L.gkeys_cap;
+        // group keys: shared memory of the CTA that finishes the row, if there is room
+        const bool keys_smem = (whole || A.cluster) && nb * 32 <= A.L.gkeys_cap;
         uint16_t* gk = keys_smem ? reinterpret_cast<uint16_t*>(smem + A.L.gkeys) : A.gkeys + (int64_t)row * (nb * 32);
+        const uint32_t rank = A.cluster ? (uint32_t)((int)blockIdx.x - row * A.slices) : 0u;
+        if (keys_smem && rank > 0) gk = cluster_map(gk, 0u);
         MassBlock* row_blocks = A.blocks + (int64_t)row * A.nblk;
         cta_sync();  // (the finish of the segment before is done with what the set-up writes)
         if (tid == 0) sh.nl = 0;
@@ -387,6 +400,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) scan_kernel(const __grid_cons
             }
         }
         first_seg = false;
+        if (A.cluster) cluster_wait();  // every CTA of the cluster has started
         ThreadStats st;
         stats_reset(st, pl.c2);
         // ---- the warp's blocks of the segment
@@ -494,7 +508,15 @@ __global__ void __launch_bounds__(kScanThreads, 2) scan_kernel(const __grid_cons
             for (int d = 16; d > 0; d >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, d);
         }
         if (lane == 0) { sh.wmax[warp] = wm; sh.wsum[warp] = ws; }
-        if (cta_sync_or(failed ? 1 : 0)) { bad = 1; break; }
+        if (cta_sync_or(failed ? 1 : 0)) {
+            bad = 1;
+            if (A.cluster) {  // (the first slice must not wait for this one for good)
+                if (tid == 0) *cluster_map(&sh.remote_fail, 0u) = 1;
+                cluster_arrive();
+                cluster_wait();
+            }
+            break;
+        }
         float m_seg = sh.wmax[0];
 #pragma unroll
         for (int w = 1; w < kScanWarps; ++w) m_seg = max_nan(m_seg, sh.wmax[w]);
@@ -512,9 +534,35 @@ __global__ void __launch_bounds__(kScanThreads, 2) scan_kernel(const __grid_cons
         src.m = m_seg; src.ls = s_seg;
         src.gkeys = gk;
         src.hist_n = hn;
+        src.remote_hist = 0;
         src.c_first = (int)blockIdx.x; src.nseg = 1;
         bool finish_here = true;
-        if (!whole) {
+        if (A.cluster) {
+            if (tid == 0) *cluster_map(&sh.part[rank], 0u) = make_float2(m_seg, s_seg);
+            if constexpr (kHist) {
+                if (rank > 0 && hn > 0) {  // history values: from the end of the first slice's list downwards
+                    const unsigned long long* list = reinterpret_cast<const unsigned long long*>(smem + A.L.list);
+                    if (tid == 0) sh.found = (int)atomicAdd(cluster_map(&sh.remote_hist, 0u), (uint32_t)hn);
+                    cta_sync();
+                    unsigned long long* dst = cluster_map(reinterpret_cast<unsigned long long*>(smem + A.L.list), 0u) + (A.L.list_cap - 1 - sh.found);
+                    for (int i = tid; i < hn; i += kThreads) dst[-i] = list[i];
+                }
+            }
+            cluster_arrive();
+            cluster_wait();
+            finish_here = rank == 0;
+            if (finish_here) {
+                if (sh.remote_fail) { bad = 1; break; }
+                src.direct = true;
+                src.remote_hist = (int)sh.remote_hist;
+                src.m = -INFINITY;
+                src.ls = 0.0f;
+                for (int s = 0; s < A.slices; ++s) src.m = max_nan(src.m, sh.part[s].x);
+                if (want_lse)
+                    for (int s = 0; s < A.slices; ++s)
+                        if (sh.part[s].y > 0.0f) src.ls += sh.part[s].y * ex2_approx(__fmul_rn(sh.part[s].x - src.m, pl.c2));
+            }
+        } else if (!whole) {
             uint8_t* rec = seg_record(A, row, (int)blockIdx.x);
             if constexpr (kHist) {
                 const unsigned long long* list = reinterpret_cast<const unsigned long long*>(smem + A.L.list);

@@ -28,5 +28,7 @@ SCAN_UNIT(bf16_hist)
 SCAN_UNIT(bf16_mask)
 SCAN_UNIT(bf16_mask_hist)
 #undef SCAN_UNIT
+// Clusters of `size` CTAs of the streaming kernel that the current device holds at once.
+cudaError_t scan_max_clusters(int size, int* count);
 
 }  // namespace born

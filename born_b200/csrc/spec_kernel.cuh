@@ -21,7 +21,7 @@
 #include <string.h>
 #include "../../include/born_sampler.h"
 #include "spec.cuh"
-#include "warp_ring.cuh"
+#include "scan_common.cuh"
 
 namespace born {
 
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kSpecThreads, 2) spec_mass_kernel(const __grid
     if (lane == 0)
         for (int s = 0; s < kSpecStages; ++s) mbar_init(reinterpret_cast<uint64_t*>(&sh.bars[s * kWarps + warp]), 1);
     mbar_fence_init();
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // (the second launch waits for this grid's end before it reads a result)
+    grid_launch_dependents();  // (the second launch waits for this grid's end before it reads a result)
     __syncwarp();
     auto row_ptr = [&](int row) {
         return reinterpret_cast<const uint8_t*>(row < ntarget ? A.target + (int64_t)row * V : A.draft + (int64_t)(row - ntarget) * V);
@@ -212,8 +212,6 @@ struct DrawShared {
     int pstat[BORN_MAX_DRAFT + 1];
     int last;
 };
-
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Sum of the draw weights of one 1024-token block, by the warp.  All loads leave before the first use.
 __device__ __forceinline__ uint64_t spec_block_sum(const DrawCtx& D, const float* rowp, const float* rowq, int tok0, int V, int vec) {
