@@ -216,8 +216,18 @@ int launch_scan(Handle* h, const ScanArgs& A, int dtype, bool aligned, int grid,
 }
 
 int launch_merge(Handle* h, const MergeArgs& M, cudaStream_t st) {
-    merge_kernel<<<M.B, kThreads, 2 * kSelCap * 8, st>>>(M);
-    CUDA_TRY(h, cudaGetLastError());
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDim = dim3((unsigned)M.B, 1, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = kWorkBytes;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    CUDA_TRY(h, cudaLaunchKernelEx(&cfg, merge_kernel, M));
     h->launches++;
     return BORN_OK;
 }

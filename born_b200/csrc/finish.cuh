@@ -48,189 +48,319 @@ struct SelectIn {
     float m_row, inv_T, u;
 };
 
-// Selection and draw over n <= kThreads candidates in shared memory (sel: rank keys, all alive;
-// selq: scratch for their masses), one candidate per thread.  The rank of a candidate is the
-// number of larger keys (keys are unique: the token index is part of them); candidates and
-// masses are then re-written in rank order, and since a mass never grows along that order the
-// kept set of every filter is a prefix of it, which every thread finds by walking the sorted
-// masses itself.  Returns false when the nucleus of S_ext is not inside the candidates (nothing is
+// Threads that share the loops over one of n <= kThreads candidates: log2.  The loops are chains of
+// shared-memory reads, so the CTA's 256 threads are dealt over (candidate, part of the loop).
+__device__ __forceinline__ int split_lg(int n) { return n <= 32 ? 3 : n <= 64 ? 2 : n <= 128 ? 1 : 0; }
+
+// Selection and draw over n <= kThreads candidates in shared memory (sel: rank keys; selq: scratch for
+// their masses and, from kThreads on, for the masses of the kept ones).  Nothing is sorted: one loop over
+// the candidates gives each its rank (the number of larger keys: keys are unique, the token index is
+// part of them) and the mass ahead of it, and since a mass never grows along the rank order the kept
+// set of every filter is a prefix of it; a second loop over the kept ones gives the mass at smaller
+// token indices.  Returns false when the nucleus of S_ext is not inside the candidates (nothing is
 // written then); all threads get the same answer.
 __device__ __forceinline__ bool select_small(const SelectIn& in, uint64_t* sel, unsigned long long* selq, ScanShared& sh,
                                              const RowOut& o) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n = in.n;
+    const int n = in.n, lg = split_lg(n), step = 1 << lg;
+    const int ci = tid >> lg, sub = tid & (step - 1);
     const int k_eff = in.k > 0 ? in.k : 0x7fffffff;
     const bool topp = in.top_p > 0.0f && in.top_p < 1.0f;
-    const bool mine = tid < n;
-    uint64_t ck = mine ? sel[tid] : 0ull;
-    int rank = 0;
-    {   // (eight broadcast loads in flight: the loop is bound by latency otherwise)
-        int j = 0;
-        for (; j + 8 <= n; j += 8) {
-            uint64_t v[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = sel[j + i];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) rank += (v[i] > ck) ? 1 : 0;
+    unsigned long long* kq = selq + kThreads;
+    if (tid < n) {
+        const uint64_t c = sel[tid];
+        uint64_t q = 0;
+        if (ck_alive(c)) {
+            const float x = scaled_shift(ck_z(c), in.m_row, in.inv_T);
+            q = (x < -30.0f) ? 0ull : mass_of(x);
+            if (in.Qa && q < in.Qa) { q = 0; sel[tid] = c & (uint64_t)kIdxMask; }  // min-p: a dead entry keeps its index only
         }
-        for (; j < n; ++j) rank += (sel[j] > ck) ? 1 : 0;
+        selq[tid] = q;
     }
-    uint64_t q = 0;
-    if (mine && rank < k_eff) {
-        const float x = scaled_shift(ck_z(ck), in.m_row, in.inv_T);
-        q = (x < -30.0f) ? 0ull : mass_of(x);
-        if (in.Qa && q < in.Qa) { q = 0; ck &= (uint64_t)kIdxMask; }  // min-p: a dead entry keeps its index only
-    }
-    cta_sync();  // every thread has read sel[] for its rank
-    const int nk = min(n, k_eff);
-    if (mine && rank < nk) { sel[rank] = ck; selq[rank] = q; }
     if (tid == 0) { sh.acc[0] = 0; sh.nw = 0; }
     cta_sync();
-    // the entry of rank `tid`, and the mass ahead of it
-    const uint64_t c2 = tid < nk ? sel[tid] : 0ull;
-    const uint64_t q2 = tid < nk ? (uint64_t)selq[tid] : 0ull;
-    uint64_t incl = q2;
+    const uint64_t ck = ci < n ? sel[ci] : 0ull;
+    const uint64_t q = ci < n ? (uint64_t)selq[ci] : 0ull;
+    int rank = 0;
+    uint64_t before = 0;
+    for (int j = sub; j < n; j += 8 * step) {  // (eight broadcast reads in flight: the loop is bound by latency otherwise)
+        uint64_t cj[8], qj[8];
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint64_t up = shfl_up_u64(incl, d);
-        if (lane >= d) incl += up;
+        for (int i = 0; i < 8; ++i) {
+            const int at = j + i * step;
+            cj[i] = at < n ? sel[at] : 0ull;
+            qj[i] = at < n ? (uint64_t)selq[at] : 0ull;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            rank += cj[i] > ck ? 1 : 0;
+            before += cj[i] > ck ? qj[i] : 0ull;
+        }
     }
-    if (lane == 31) sh.red64[warp] = incl;
+    for (int d = 1; d < step; d <<= 1) {
+        rank += __shfl_xor_sync(0xffffffffu, rank, d);
+        before += shfl_xor_u64(before, d);
+    }
+    const bool first = sub == 0 && ci < n;
+    const bool in_k = ck_alive(ck) && rank < k_eff;
+    bool kept = in_k;
+    uint64_t w = (first && in_k) ? q : 0ull;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) w += shfl_xor_u64(w, d);
+    if (lane == 0) sh.red64[warp] = w;
+    if (!topp) {
+        if (first) kq[ci] = in_k ? q : 0ull;
+        const uint32_t kb = __ballot_sync(0xffffffffu, first && in_k);
+        if (lane == 0 && kb) smem_red_add(&sh.nw, (uint32_t)__popc(kb));
+    }
     cta_sync();
-    uint64_t off = 0, tot = 0;
+    uint64_t S = 0;
 #pragma unroll
-    for (int w = 0; w < kScanWarps; ++w) {
-        const uint64_t x = sh.red64[w];
-        if (w < warp) off += x;
-        tot += x;
-    }
-    const uint64_t before = off + incl - q2;
-    uint64_t Tp = ~0ull;
+    for (int i = 0; i < kScanWarps; ++i) S += sh.red64[i];
     if (topp) {
-        Tp = __double2ull_rz(__dmul_rn((double)in.top_p, __ull2double_rn(in.S_ext ? in.S_ext : tot)));
+        // kept: the mass ahead still short of the nucleus; the one that completes it reports the sum
+        uint64_t Tp = __double2ull_rz(__dmul_rn((double)in.top_p, __ull2double_rn(in.S_ext ? in.S_ext : S)));
         if (Tp < 1) Tp = 1;
+        kept = in_k && before < Tp;
+        if (first) kq[ci] = kept ? q : 0ull;
+        if (first && kept && before + q >= Tp) sh.acc[0] = before + q;
+        const uint32_t kb = __ballot_sync(0xffffffffu, first && kept);
+        if (lane == 0 && kb) smem_red_add(&sh.nw, (uint32_t)__popc(kb));
+        cta_sync();
+        S = sh.acc[0];
+        if (in.S_ext && S < Tp) return false;  // (uniform)
     }
-    // kept: alive and the mass ahead still short of the nucleus -- a prefix of the rank order;
-    // its last entry of every warp reports the prefix's length and mass
-    const bool kept = tid < nk && ck_alive(c2) && before < Tp;
-    const uint32_t kb = __ballot_sync(0xffffffffu, kept);
-    if (kb && lane == 31 - __clz(kb)) {
-        atomicMax(&sh.nw, tid + 1);
-        atomicMax(&sh.acc[0], (unsigned long long)(before + q2));
-    }
-    cta_sync();
-    const int R = sh.nw;
-    const uint64_t S = sh.acc[0];
-    if (topp && in.S_ext && S < Tp) return false;  // (uniform)
     if (S == 0) {  // cannot happen while the row maximum is finite; never divide by it
         row_fail(o, BORN_ROW_ALL_MASKED);
         return true;
     }
     uint64_t t = __double2ull_rz(__dmul_rn((double)in.u, __ull2double_rn(S)));
     if (t > S - 1) t = S - 1;
-    if (tid < R) {
-        const uint32_t my_low = (uint32_t)(c2 & kIdxMask);  // larger low bits = smaller token index
-        uint64_t pre = 0;
-        int j = 0;
-        for (; j + 8 <= R; j += 8) {
-            uint64_t cj[8], qj[8];
+    const uint32_t my_low = (uint32_t)(ck & kIdxMask);  // larger low bits = smaller token index
+    uint64_t pre = 0;
+    for (int j = sub; j < n; j += 8 * step) {
+        uint32_t lj[8];
+        uint64_t qj[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) { cj[i] = sel[j + i]; qj[i] = selq[j + i]; }
+        for (int i = 0; i < 8; ++i) {
+            const int at = j + i * step;
+            lj[i] = at < n ? (uint32_t)sel[at] & kIdxMask : 0u;
+            qj[i] = at < n ? (uint64_t)kq[at] : 0ull;
+        }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) pre += ((uint32_t)(cj[i] & kIdxMask) > my_low) ? qj[i] : 0ull;
-        }
-        for (; j < R; ++j) pre += ((uint32_t)(sel[j] & kIdxMask) > my_low) ? (uint64_t)selq[j] : 0ull;
-        if (pre <= t && t < pre + q2) {
-            o.token[o.row] = ck_idx(c2);
-            o.status[o.row] = BORN_ROW_OK;
-            if (o.prob) o.prob[o.row] = __double2float_rn(__ddiv_rn(__ull2double_rn(q2), __ull2double_rn(S)));
-        }
-        if (o.kept_ids && tid < o.kept_stride) o.kept_ids[(int64_t)o.row * o.kept_stride + tid] = ck_idx(c2);
+        for (int i = 0; i < 8; ++i) pre += lj[i] > my_low ? qj[i] : 0ull;
     }
-    if (o.kept_count && tid == 0) o.kept_count[o.row] = R;
+    for (int d = 1; d < step; d <<= 1) pre += shfl_xor_u64(pre, d);
+    if (first && kept) {
+        if (pre <= t && t < pre + q) {
+            o.token[o.row] = ck_idx(ck);
+            o.status[o.row] = BORN_ROW_OK;
+            if (o.prob) o.prob[o.row] = __double2float_rn(__ddiv_rn(__ull2double_rn(q), __ull2double_rn(S)));
+        }
+        if (o.kept_ids && rank < o.kept_stride) o.kept_ids[(int64_t)o.row * o.kept_stride + rank] = ck_idx(ck);
+    }
+    if (o.kept_count && tid == 0) o.kept_count[o.row] = sh.nw;
     return true;
 }
 
-// Selection and draw over kThreads < n <= kSelCap candidates: radix select, then mass-weighted
-// radix threshold searches.  Same rules as select_small.
-static __device__ __noinline__ bool select_and_draw(const SelectIn in, uint64_t* sel, unsigned long long* selq, ScanShared& sh,
-                                             const RowOut o) {
-    const int tid = threadIdx.x;
+// First bin at which the running total of `total_of(bin)` exceeds `target`, the total ahead of it in
+// `before`; -1 when the whole total does not.  All threads get the same answer.  (The caller's last
+// barrier covers the bins.)
+template <typename F>
+__device__ __forceinline__ int find_bin(F total_of, unsigned long long target, unsigned long long& before, ScanShared& sh) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int PER = kBins / kThreads;
+    uint64_t w[PER], loc = 0;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) { w[j] = total_of(PER * tid + j); loc += w[j]; }
+    uint64_t incl = loc;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint64_t up = shfl_up_u64(incl, d);
+        if (lane >= d) incl += up;
+    }
+    if (lane == 31) sh.red64[warp] = incl;
+    if (tid == 0) sh.found = -1;
+    cta_sync();
+    for (int i = 0; i < warp; ++i) incl += sh.red64[i];
+    if (incl > target && incl - loc <= target) {
+        uint64_t acc = incl - loc;
+        int j = 0;
+        for (; j < PER - 1 && acc + w[j] <= target; ++j) acc += w[j];
+        sh.found = PER * tid + j;
+        sh.before = acc;
+    }
+    cta_sync();
+    before = sh.before;
+    return sh.found;
+}
+
+// Selection and draw over kThreads < n <= kSelCap candidates, the same rules, four candidates per thread.
+// A counting sort puts them in rank order: bins of equal width in value from the best candidate down,
+// places inside a bin by comparison.  Then the masses are scanned in rank order, and the draw finds its
+// token through bins of the token index.  (Three radix descents, over keys, masses and indices, took
+// 18 us for 300 candidates.)  `bins`: kBins 64-bit words.
+static __device__ __noinline__ bool select_large(const SelectIn in, uint64_t* sel, unsigned long long* selq, uint32_t* bins,
+                                                 ScanShared& sh, const RowOut o) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = in.n;
     const int k_eff = in.k > 0 ? in.k : 0x7fffffff;
     const bool topp = in.top_p > 0.0f && in.top_p < 1.0f;
+    constexpr int PER = kSelCap / kThreads;
+    static_assert(PER == 4 && kBins == 4 * kThreads, "four candidates and four bins per thread");
     cta_sync();
-    // ---- large set: radix select, then mass-weighted radix threshold searches
-    if (n > k_eff) {
-        const uint64_t T = block_radix_search<true, 56, true>(
-            n, (unsigned long long)(k_eff - 1), [&](int i) { return sel[i]; }, [&](int) { return 1ull; }, sh.sc);
-        for (int i = tid; i < n; i += kThreads)
-            if (sel[i] < T) sel[i] &= (uint64_t)kIdxMask;
-        cta_sync();
+    // ---- ranges of the values and of the indices
+    uint64_t c[PER];
+    uint32_t zlo = 0xFFFFFFFFu, zhi = 0u, ilo = 0xFFFFFFFFu, ihi = 0u;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int i = tid + j * kThreads;
+        c[j] = i < n ? sel[i] : 0ull;
+        if (!ck_alive(c[j])) continue;
+        const uint32_t z = (uint32_t)(c[j] >> 24), low = (uint32_t)c[j] & kIdxMask;
+        zlo = min(zlo, z); zhi = max(zhi, z);
+        ilo = min(ilo, low); ihi = max(ihi, low);
     }
-    for (int i = tid; i < n; i += kThreads) {
-        const uint64_t c = sel[i];
-        uint64_t q = 0;
-        if (ck_alive(c)) {
-            const float x = scaled_shift(ck_z(c), in.m_row, in.inv_T);
-            q = (x < -30.0f) ? 0ull : mass_of(x);
-            if (in.Qa && q < in.Qa) { q = 0; sel[i] = c & (uint64_t)kIdxMask; }
+    zlo = __reduce_min_sync(0xffffffffu, zlo); zhi = __reduce_max_sync(0xffffffffu, zhi);
+    ilo = __reduce_min_sync(0xffffffffu, ilo); ihi = __reduce_max_sync(0xffffffffu, ihi);
+    if (lane == 0) { sh.sc.c[4 * warp] = zlo; sh.sc.c[4 * warp + 1] = zhi; sh.sc.c[4 * warp + 2] = ilo; sh.sc.c[4 * warp + 3] = ihi; }
+    reinterpret_cast<uint4*>(bins)[tid] = make_uint4(0u, 0u, 0u, 0u);
+    if (tid == 0) { sh.acc[0] = 0; sh.nw = 0; sh.nl = 0; }
+    cta_sync();
+#pragma unroll
+    for (int w = 0; w < kScanWarps; ++w) {
+        zlo = min(zlo, sh.sc.c[4 * w]); zhi = max(zhi, sh.sc.c[4 * w + 1]);
+        ilo = min(ilo, sh.sc.c[4 * w + 2]); ihi = max(ihi, sh.sc.c[4 * w + 3]);
+    }
+    // ---- counting sort (the bin never falls as the value falls; dead entries go last: their keys are the smallest)
+    const float top = zkey_to_float(zhi), span = top - zkey_to_float(zlo);
+    const float scale = span > 0.0f ? (float)(kBins - 1) / span : 0.0f;
+    int bin[PER];
+    uint32_t pos[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        bin[j] = ck_alive(c[j]) ? (int)fminf(__fmul_rn(top - ck_z(c[j]), scale), (float)(kBins - 1)) : kBins - 1;
+        pos[j] = tid + j * kThreads < n ? smem_atom_add(&bins[bin[j]], 1u) : 0u;
+    }
+    cta_sync();
+    const uint4 cnt = reinterpret_cast<const uint4*>(bins)[tid];
+    uint32_t incl = cnt.x + cnt.y + cnt.z + cnt.w;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += up;
+    }
+    if (lane == 31) sh.redu[warp] = incl;
+    cta_sync();
+    for (int w = 0; w < warp; ++w) incl += sh.redu[w];
+    const uint32_t o3 = incl - cnt.w, o2 = o3 - cnt.z, o1 = o2 - cnt.y;
+    reinterpret_cast<uint4*>(bins)[tid] = make_uint4(o1 - cnt.x, o1, o2, o3);
+    cta_sync();
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+        if (tid + j * kThreads < n) selq[bins[bin[j]] + pos[j]] = c[j];
+    cta_sync();
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        if (tid + j * kThreads >= n) continue;
+        const int b0 = (int)bins[bin[j]], b1 = bin[j] + 1 < kBins ? (int)bins[bin[j] + 1] : n;
+        int r = b0;
+        for (int i = b0; i < b1; ++i) r += selq[i] > c[j] ? 1 : 0;
+        sel[r] = c[j];
+    }
+    cta_sync();
+    // ---- masses in rank order (four consecutive ranks per thread), kept prefix
+    uint64_t q[PER], loc = 0;
+    bool kept[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int r = PER * tid + j;
+        c[j] = r < n ? sel[r] : 0ull;
+        q[j] = 0;
+        kept[j] = ck_alive(c[j]) && r < k_eff;
+        if (kept[j]) {
+            const float x = scaled_shift(ck_z(c[j]), in.m_row, in.inv_T);
+            q[j] = (x < -30.0f) ? 0ull : mass_of(x);
+            if (in.Qa && q[j] < in.Qa) { q[j] = 0; kept[j] = false; }
         }
-        selq[i] = q;
+        loc += q[j];
     }
+    uint64_t run = loc;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint64_t up = shfl_up_u64(run, d);
+        if (lane >= d) run += up;
+    }
+    if (lane == 31) sh.red64[warp] = run;
+    unsigned long long* ibins = reinterpret_cast<unsigned long long*>(bins);
+    reinterpret_cast<uint4*>(bins)[tid] = make_uint4(0u, 0u, 0u, 0u);
+    reinterpret_cast<uint4*>(bins)[tid + kThreads] = make_uint4(0u, 0u, 0u, 0u);
+    cta_sync();
+    uint64_t S = 0;
+    run -= loc;
+#pragma unroll
+    for (int w = 0; w < kScanWarps; ++w) {
+        if (w < warp) run += sh.red64[w];
+        S += sh.red64[w];
+    }
+    uint64_t Tp = ~0ull;
+    if (topp) {
+        Tp = __double2ull_rz(__dmul_rn((double)in.top_p, __ull2double_rn(in.S_ext ? in.S_ext : S)));
+        if (Tp < 1) Tp = 1;
+    }
+    const int sft = max(0, 22 - __clz((int)(ihi - ilo)));  // (the index range is below 2^24: at most kBins bins)
+    int nkept = 0;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        kept[j] = kept[j] && run < Tp;
+        nkept += kept[j] ? 1 : 0;
+        if (topp && kept[j] && run + q[j] >= Tp) sh.acc[0] = run + q[j];
+        run += q[j];
+        if (!kept[j]) q[j] = 0;
+        bin[j] = (int)((ihi - ((uint32_t)c[j] & kIdxMask)) >> sft);  // larger low bits = smaller token index
+        if (q[j]) atomicAdd(&ibins[bin[j]], (unsigned long long)q[j]);
+    }
+    nkept = __reduce_add_sync(0xffffffffu, nkept);
+    if (lane == 0 && nkept) smem_red_add(&sh.nw, (uint32_t)nkept);
     cta_sync();
     if (topp) {
-        uint64_t part = 0;
-        for (int i = tid; i < n; i += kThreads) part += selq[i];
-        const uint64_t S = block_sum_u64(part, sh.red64);
-        uint64_t Tp = __double2ull_rz(__dmul_rn((double)in.top_p, __ull2double_rn(in.S_ext ? in.S_ext : S)));
-        if (Tp < 1) Tp = 1;
-        if (in.S_ext && S < Tp) return false;
-        if (S >= Tp) {
-            // dead entries take part with weight 0 (their keys are unique small numbers)
-            const uint64_t C = block_radix_search<true, 56, false>(
-                n, Tp - 1, [&](int i) { return sel[i]; }, [&](int i) { return selq[i]; }, sh.sc);
-            for (int i = tid; i < n; i += kThreads)
-                if (sel[i] < C && ck_alive(sel[i])) { selq[i] = 0; sel[i] &= (uint64_t)kIdxMask; }
-            cta_sync();
-        }
+        S = sh.acc[0];
+        if (in.S_ext && S < Tp) return false;  // (uniform)
     }
-    uint64_t part = 0;
-    for (int i = tid; i < n; i += kThreads) part += selq[i];
-    const uint64_t S = block_sum_u64(part, sh.red64);
+    const int R = sh.nw;
     if (S == 0) {
         row_fail(o, BORN_ROW_ALL_MASKED);
         return true;
     }
+    // ---- the draw: the bin of the index that holds t, then its members by comparison
     uint64_t t = __double2ull_rz(__dmul_rn((double)in.u, __ull2double_rn(S)));
     if (t > S - 1) t = S - 1;
-    // walk in ascending token index: key = index; dead entries weigh nothing but need unique keys
-    const uint64_t tok64 = block_radix_search<false, 25, false>(
-        n, t, [&](int i) { return ck_alive(sel[i]) ? (uint64_t)ck_idx(sel[i]) : ((1ull << 24) | (uint64_t)i); },
-        [&](int i) { return selq[i]; }, sh.sc);
-    const int tok = (int)tok64;
-    for (int i = tid; i < n; i += kThreads) {
-        if (ck_alive(sel[i]) && ck_idx(sel[i]) == tok) {
-            o.token[o.row] = tok;
-            o.status[o.row] = BORN_ROW_OK;
-            if (o.prob) o.prob[o.row] = __double2float_rn(__ddiv_rn(__ull2double_rn(selq[i]), __ull2double_rn(S)));
-        }
+    unsigned long long before;
+    const int hit = find_bin([&](int i) { return (uint64_t)ibins[i]; }, t, before, sh);
+    const uint32_t rel_mask = (1u << sft) - 1u;  // sft <= 14, and a mass has 41 bits
+    uint32_t rel[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        rel[j] = (ihi - ((uint32_t)c[j] & kIdxMask)) & rel_mask;
+        if (q[j] && bin[j] == hit) ibins[smem_atom_add(&sh.nl, 1u)] = (q[j] << 14) | rel[j];
     }
-    if (o.kept_count || o.kept_ids) {
-        int alive = 0;
-        for (int i = tid; i < n; i += kThreads) {
-            const uint64_t c = sel[i];
-            if (!ck_alive(c)) continue;
-            ++alive;
-            if (o.kept_ids) {
-                int rank = 0;
-                for (int j = 0; j < n; ++j) rank += (sel[j] > c) ? 1 : 0;
-                if (rank < o.kept_stride) o.kept_ids[(int64_t)o.row * o.kept_stride + rank] = ck_idx(c);
+    cta_sync();
+    const int nb = sh.nl;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        if (q[j] && bin[j] == hit) {
+            uint64_t pre = before;
+            for (int i = 0; i < nb; ++i) pre += ((uint32_t)ibins[i] & 0x3FFFu) < rel[j] ? (uint64_t)(ibins[i] >> 14) : 0ull;
+            if (pre <= t && t < pre + q[j]) {
+                o.token[o.row] = ck_idx(c[j]);
+                o.status[o.row] = BORN_ROW_OK;
+                if (o.prob) o.prob[o.row] = __double2float_rn(__ddiv_rn(__ull2double_rn(q[j]), __ull2double_rn(S)));
             }
         }
-        const uint64_t tot = block_sum_u64((uint64_t)alive, sh.red64);
-        if (tid == 0 && o.kept_count) o.kept_count[o.row] = (int)tot;
+        const int r = PER * tid + j;
+        if (o.kept_ids && kept[j] && r < o.kept_stride) o.kept_ids[(int64_t)o.row * o.kept_stride + r] = ck_idx(c[j]);
     }
+    if (o.kept_count && tid == 0) o.kept_count[o.row] = R;
     return true;
 }
 
@@ -398,38 +528,6 @@ __device__ __forceinline__ void bin_mass(uint32_t* limb, int bin, uint64_t q) {
 __device__ __forceinline__ uint64_t bin_total(const uint32_t* limb, int bin) {
     return (uint64_t)limb[bin] + ((uint64_t)limb[kBins + bin] << 14) + ((uint64_t)limb[2 * kBins + bin] << 28);
 }
-// First bin at which the running total of `total_of(bin)` exceeds `target`, the total ahead of it in
-// `before`; -1 when the whole total does not.  All threads get the same answer.  (The caller's last
-// barrier covers the bins.)
-template <typename F>
-__device__ __forceinline__ int find_bin(F total_of, unsigned long long target, unsigned long long& before, ScanShared& sh) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int PER = kBins / kThreads;
-    uint64_t w[PER], loc = 0;
-#pragma unroll
-    for (int j = 0; j < PER; ++j) { w[j] = total_of(PER * tid + j); loc += w[j]; }
-    uint64_t incl = loc;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint64_t up = shfl_up_u64(incl, d);
-        if (lane >= d) incl += up;
-    }
-    if (lane == 31) sh.red64[warp] = incl;
-    if (tid == 0) sh.found = -1;
-    cta_sync();
-    for (int i = 0; i < warp; ++i) incl += sh.red64[i];
-    if (incl > target && incl - loc <= target) {
-        uint64_t acc = incl - loc;
-        int j = 0;
-        for (; j < PER - 1 && acc + w[j] <= target; ++j) acc += w[j];
-        sh.found = PER * tid + j;
-        sh.before = acc;
-    }
-    cta_sync();
-    before = sh.before;
-    return sh.found;
-}
-
 // A completed row: where its statistics, group keys and history values are.
 struct RowSrc {
     int row, b, g;               // virtual row; caller row and vocabulary segment
@@ -452,31 +550,62 @@ __device__ __forceinline__ void defer_row(const ScanArgs& A, ScanShared& sh, int
     if (A.slices == 0) A.deferred[row] = word;
 }
 
-// The k-th largest of n 16-bit keys (key_of(i), zero: none), from above, as far as the bins resolve
-// it: a key that at least k of them reach, and not many more.  Keys below the smallest of the threads'
-// own maxima cannot matter (at least as many reach that as there are threads; for small k, pairs or
-// quartets of threads), so the bins -- equal steps of the value below the maximum m -- only span what is
-// left.  All threads get the same answer; kDeadKey16 + 1 when fewer than k are alive.
+// A key that at least k of the n 16-bit keys (key_of(i), zero: none) reach, and not many more.  Up to
+// half as many as there are threads: the k-th largest of the threads' own maxima -- k keys reach it, and
+// few more, since the k best seldom share a thread (50 of 4008 keys: 54 reach it).  Every warp holds all
+// 256 maxima and finds it by bisection, so one barrier is enough (bins over all keys, the way of larger k,
+// take four and 2.3 us).
+// Larger k, or too few threads with a live key: bins -- equal steps of the value below the maximum m --
+// down to the smallest of the threads' maxima (at least as many keys as threads reach that).  All
+// threads get the same answer; kDeadKey16 + 1 when fewer than k are alive.
 template <typename F>
 __device__ __forceinline__ uint32_t kth_key(F key_of, int n, int k, float m, uint32_t* bins, ScanShared& sh) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int kReg = 16;  // keys a thread keeps in registers: 4096 in all
     uint32_t kk[kReg];
-    uint32_t mx = 0, mn = 0xFFFFu;
-    auto see = [&](uint32_t key) {
-        mx = max(mx, key);
-        mn = min(mn, key > kDeadKey16 ? key : 0xFFFFu);
-    };
+    uint32_t mx = 0;
 #pragma unroll
     for (int i = 0; i < kReg; ++i) {
         const int g = tid + i * kThreads;
         kk[i] = g < n ? key_of(g) : 0u;
     }
 #pragma unroll
+    for (int i = 0; i < kReg; ++i) mx = max(mx, kk[i]);
+    for (int g = tid + kReg * kThreads; g < n; g += kThreads) mx = max(mx, key_of(g));
+    if (k <= kThreads / 2) {
+        uint16_t* maxima = reinterpret_cast<uint16_t*>(sh.sc.c);
+        maxima[tid] = (uint16_t)mx;
+        cta_sync();
+        const uint4 w = reinterpret_cast<const uint4*>(maxima)[lane];
+        const uint32_t v[8] = {w.x & 0xFFFFu, w.x >> 16, w.y & 0xFFFFu, w.y >> 16, w.z & 0xFFFFu, w.z >> 16, w.w & 0xFFFFu, w.w >> 16};
+        auto reach = [&](uint32_t key) {
+            int c = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) c += v[i] >= key ? 1 : 0;
+            return __reduce_add_sync(0xffffffffu, c);
+        };
+        uint32_t lo = kDeadKey16 + 1u;
+        if (reach(lo) >= k) {
+            uint32_t hi = v[0], mn = v[0];
+#pragma unroll
+            for (int i = 1; i < 8; ++i) { hi = max(hi, v[i]); mn = min(mn, v[i]); }
+            hi = __reduce_max_sync(0xffffffffu, hi) + 1u;
+            lo = max(lo, __reduce_min_sync(0xffffffffu, mn));
+            while (hi - lo > 1u) {  // k of the maxima reach lo, fewer reach hi
+                const uint32_t mid = (lo + hi) >> 1;
+                const int c = reach(mid);
+                if (c >= k) lo = mid;
+                else hi = mid;
+                if (c >= k && c <= k + k / 16) break;
+            }
+            return lo;
+        }
+    }
+    uint32_t mn = 0xFFFFu;
+    auto see = [&](uint32_t key) { mn = min(mn, key > kDeadKey16 ? key : 0xFFFFu); };
+#pragma unroll
     for (int i = 0; i < kReg; ++i) see(kk[i]);
     for (int g = tid + kReg * kThreads; g < n; g += kThreads) see(key_of(g));
-    if (k <= kThreads / 2) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    if (k <= kThreads / 4) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
     const uint32_t lo_w = __reduce_min_sync(0xffffffffu, mx), mn_w = __reduce_min_sync(0xffffffffu, mn);
     if (lane == 0) sh.redu[warp] = (lo_w << 16) | mn_w;
     reinterpret_cast<uint4*>(bins)[tid] = make_uint4(0u, 0u, 0u, 0u);
@@ -538,23 +667,48 @@ __device__ __forceinline__ float raw_logit(const uint8_t* base, int tok) {
 }
 
 // Every group of the row whose key reaches `tk`, read again: f(tok, z) with eight groups at a time, a
-// lane per token (z = -inf where there is none, or the mask hides it; no penalties).  A warp lists
-// the groups it finds among its share of the keys first, so that the re-reads leave eight at a time.
+// lane per token (z = -inf where there is none, or the mask hides it; no penalties).  The CTA lists
+// the groups it finds, 4096 keys a round, and deals them over its warps eight at a time: each warp has
+// one round of reads in flight as long as there are no more than 64 groups.  (Lists per warp left some
+// warps with two rounds, a microsecond apart.)  sh.ng is zero on entry; the caller's next barrier
+// frees the list.
 template <typename T, typename F>
-__device__ __forceinline__ void for_groups(const ScanArgs& A, const uint16_t* keys, int b, int g, uint32_t tk, uint32_t* wl, F f) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+__device__ __forceinline__ void for_groups(const ScanArgs& A, ScanShared& sh, const uint16_t* keys, int b, int g, uint32_t tk, uint16_t* list,
+                                           F f) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ngrp = (A.V + kGrpTok - 1) / kGrpTok;
     const uint8_t* base = reinterpret_cast<const uint8_t*>(A.logits) + ((int64_t)b * A.row_stride + (int64_t)g * A.V) * (int64_t)sizeof(T);
     const uint32_t* mrow = A.mask ? A.mask + (int64_t)b * A.mask_stride : nullptr;
-    uint32_t* list = wl + warp * kGrpList;
-    int n = 0;
-    auto flush = [&]() {
-        __syncwarp();
-        for (int i = 0; i < n; i += 8) {
+    constexpr int kPer = kGrpRound / kThreads;
+    int round = 0;
+    for (int g0 = 0; g0 < ngrp; g0 += kGrpRound, round ^= 1) {
+        uint32_t hits = 0;
+#pragma unroll
+        for (int e = 0; e < kPer; ++e) {
+            const int gi = g0 + e * kThreads + tid;
+            const uint32_t key = gi < ngrp ? (uint32_t)keys[gi] : 0u;
+            hits |= key >= tk ? 1u << e : 0u;
+        }
+        if (__any_sync(0xffffffffu, hits != 0)) {
+            uint32_t incl = (uint32_t)__popc(hits);
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t up = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += up;
+            }
+            uint32_t at = 0;
+            if (lane == 31) at = smem_atom_add(&sh.ng[round], incl);
+            at = __shfl_sync(0xffffffffu, at, 31) + incl - (uint32_t)__popc(hits);
+            for (; hits; hits &= hits - 1u) list[at++] = (uint16_t)((__ffs(hits) - 1) * kThreads + tid);
+        }
+        cta_sync();
+        const int n = (int)sh.ng[round];
+        if (tid == 0) sh.ng[round ^ 1] = 0;
+        for (int i = warp * 8; i < n; i += kScanWarps * 8) {
             int tok[8];
             float z[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) tok[e] = i + e < n ? (int)list[i + e] * kGrpTok + lane : A.V;
+            for (int e = 0; e < 8; ++e) tok[e] = i + e < n ? (g0 + (int)list[i + e]) * kGrpTok + lane : A.V;
 #pragma unroll
             for (int e = 0; e < 8; ++e) z[e] = tok[e] < A.V ? raw_logit<T>(base, tok[e]) : -INFINITY;
             if (mrow) {
@@ -566,26 +720,8 @@ __device__ __forceinline__ void for_groups(const ScanArgs& A, const uint16_t* ke
             }
             f(tok, z);
         }
-        __syncwarp();
-        n = 0;
-    };
-    for (int base_g = warp * 32; base_g < ngrp; base_g += 4 * kThreads) {
-        uint32_t key[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int gi = base_g + e * kThreads + lane;
-            key[e] = gi < ngrp ? (keys ? (uint32_t)keys[gi] : 0xFFFFu) : 0u;
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const bool hit = key[e] >= tk;
-            const uint32_t hb = __ballot_sync(0xffffffffu, hit);
-            if (hit) list[n + __popc(hb & ((1u << lane) - 1u))] = (uint32_t)(base_g + e * kThreads + lane);
-            n += __popc(hb);
-        }
-        if (n > kGrpList - 128) flush();
+        if (g0 + kGrpRound < ngrp) cta_sync();
     }
-    if (n) flush();
 }
 
 // The row's history values: f(token of the virtual row, penalised value) for every entry, dealt over
@@ -636,14 +772,18 @@ __device__ __forceinline__ uint32_t kth_token_key(const ScanArgs& A, const RowSr
 // Every token of the row at or above tau into sel (rank keys); returns their number, which may exceed
 // kSelCap (what does not fit is dropped: the caller looks at the number).  sh.nl is zero on entry.
 // A history token's raw value is struck out (its key keeps the index only, so that keys stay
-// unique) and its penalised value added.
+// unique) and its penalised value added.  The candidates leave a bit each in a 4096-bit map of
+// (token mod 4096), so that only the few history tokens that may be candidates look for themselves
+// among them (every one of 512 comparing itself with 50 candidates took 1.5 us).
 template <typename T, bool kHist>
 __device__ __forceinline__ int gather_row(const ScanArgs& A, ScanShared& sh, const uint8_t* smem, const RowSrc& src, float tau, uint64_t* sel,
-                                          uint32_t* wl) {
+                                          uint16_t* wl) {
     const int lane = threadIdx.x & 31;
     const float tf = fmaxf(tau, -FLT_MAX);
     const int id0 = A.idx_base + src.g * A.V;
-    for_groups<T>(A, src.gkeys, src.b, src.g, zkey(tf) >> 16, wl, [&](const int (&tok)[8], const float (&z)[8]) {
+    uint32_t* seen = reinterpret_cast<uint32_t*>(sh.bcnt);
+    const bool strike = kHist && penalties_on(src.rp);
+    for_groups<T>(A, sh, src.gkeys, src.b, src.g, zkey(tf) >> 16, wl, [&](const int (&tok)[8], const float (&z)[8]) {
         uint32_t hb[8], sum = 0;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
@@ -657,27 +797,29 @@ __device__ __forceinline__ int gather_row(const ScanArgs& A, ScanShared& sh, con
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const uint32_t at = pos + __popc(hb[e] & ((1u << lane) - 1u));
-            if (z[e] >= tf && at < (uint32_t)kSelCap) sel[at] = make_ck(z[e], id0 + tok[e]);
+            if (z[e] >= tf && at < (uint32_t)kSelCap) {
+                sel[at] = make_ck(z[e], id0 + tok[e]);
+                if (strike) smem_red_or(&seen[((uint32_t)tok[e] >> 5) & 127u], 1u << (tok[e] & 31));
+            }
             pos += __popc(hb[e]);
         }
     });
     cta_sync();
     int n = sh.nl;
     if constexpr (kHist) {
-        if (penalties_on(src.rp) && n <= kSelCap) {
-            for_history(A, smem, src, [&](int tok, float) {
-                const uint32_t low = kIdxMask - (uint32_t)(id0 + tok);
-                for (int i = 0; i < n; ++i)
-                    if ((uint32_t)(sel[i] & kIdxMask) == low) sel[i] = low;
-            });
-            cta_sync();
+        if (strike && n <= kSelCap) {
             for_history(A, smem, src, [&](int tok, float zp) {
+                if ((seen[((uint32_t)tok >> 5) & 127u] >> (tok & 31)) & 1u) {
+                    const uint32_t low = kIdxMask - (uint32_t)(id0 + tok);
+                    for (int i = 0; i < n; ++i)
+                        if ((uint32_t)(sel[i] & kIdxMask) == low) sel[i] = low;
+                }
                 if (!(zp >= tf)) return;
-                const uint32_t pos = smem_atom_add(&sh.nl, 1u);
+                const uint32_t pos = (uint32_t)n + smem_atom_add(&sh.nh, 1u);
                 if (pos < (uint32_t)kSelCap) sel[pos] = make_ck(zp, id0 + tok);
             });
             cta_sync();
-            n = sh.nl;
+            n += (int)sh.nh;
         }
     }
     return n;
@@ -705,22 +847,20 @@ __device__ __forceinline__ void write_packed(const ScanArgs& A, ScanShared& sh, 
     uint8_t* rec = A.packed + (int64_t)g * A.packed_seg_stride + (int64_t)b * A.packed_row_stride;
     uint64_t* ent = reinterpret_cast<uint64_t*>(rec + kRecordHdrBytes);
     if (n > kThreads) n = cut_to_k(sel, tmp, n, k, sh);
-    const uint64_t ck = tid < n ? sel[tid] : 0ull;
-    const int alive = cta_sync_count(tid < n && ck_alive(ck));
+    const int lg = split_lg(n), step = 1 << lg, ci = tid >> lg, sub = tid & (step - 1);
+    const uint64_t ck = ci < n ? sel[ci] : 0ull;
+    const int alive = cta_sync_count(sub == 0 && ck_alive(ck));
     int rank = 0;
-    {
-        int j = 0;
-        for (; j + 8 <= n; j += 8) {
-            uint64_t v[8];
+    for (int j = sub; j < n; j += 8 * step) {
+        uint64_t v[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = sel[j + i];
+        for (int i = 0; i < 8; ++i) v[i] = j + i * step < n ? sel[j + i * step] : 0ull;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) rank += (v[i] > ck) ? 1 : 0;
-        }
-        for (; j < n; ++j) rank += (sel[j] > ck) ? 1 : 0;
+        for (int i = 0; i < 8; ++i) rank += (v[i] > ck) ? 1 : 0;
     }
+    for (int d = 1; d < step; d <<= 1) rank += __shfl_xor_sync(0xffffffffu, rank, d);
     const int nk = min(alive, k);
-    if (tid < n && rank < nk) ent[rank] = ck;
+    if (sub == 0 && ci < n && rank < nk) ent[rank] = ck;
     if (tid == 0) {
         PackedHdr h;
         h.m = m; h.lse_s = lse_s; h.count = (uint32_t)nk;
@@ -744,7 +884,7 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
     const bool mass = RouteOf<kRoute>::mass && (!RouteOf<kRoute>::cand || pl.need_mass);
     uint64_t* sel = reinterpret_cast<uint64_t*>(smem + A.L.work);
     unsigned long long* selq = reinterpret_cast<unsigned long long*>(sel + kSelCap);
-    uint32_t* wl = reinterpret_cast<uint32_t*>(selq + kSelCap);
+    uint16_t* wl = reinterpret_cast<uint16_t*>(selq + kSelCap);  // group list; bins of the larger selection
     const int ngrp = (A.V + kGrpTok - 1) / kGrpTok;
 
     float m = src.m, ls = src.ls;
@@ -857,7 +997,7 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
                     if (k1 >= ck16) bin_mass(limb, nucleus_bin(z1, m, pl.inv_T), q1);
                 }
             } else {
-                for_groups<T>(A, src.gkeys, b, g, zkey(cut) >> 16, wl, [&](const int (&)[8], const float (&z)[8]) {
+                for_groups<T>(A, sh, src.gkeys, b, g, zkey(cut) >> 16, wl, [&](const int (&)[8], const float (&z)[8]) {
 #pragma unroll
                     for (int e = 0; e < 8; e += 2) {
                         uint64_t q[2];
@@ -869,6 +1009,7 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
                 });
             }
             cta_sync();
+            if (tid == 0) sh.ng[0] = sh.ng[1] = 0;  // (for the candidates' own round)
             bin = find_bin([&](int i) { return bin_total(limb, i); }, Tp - 1, before, sh);
             cta_sync();
         }
@@ -886,7 +1027,7 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
             tau = fmaxf(tau, zkey_to_float(tk << 16));
         }
     }
-    int n = gather_row<T, kHist>(A, sh, smem, src, tau, sel, wl);
+    const int n = gather_row<T, kHist>(A, sh, smem, src, tau, sel, wl);
     if (n > kSelCap) {
         if (tid == 0) defer_row(A, sh, row, mass ? 7u : pl.k > 0 ? 5u : pl.greedy ? 1u : 6u);
         return;
@@ -909,7 +1050,6 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
         }
         return;
     }
-    if (pl.k > 0 && pl.k <= kThreads && n > kThreads) n = cut_to_k(sel, reinterpret_cast<uint64_t*>(selq), n, pl.k, sh);
     SelectIn in;
     in.n = n;
     in.k = pl.k;
@@ -917,7 +1057,7 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
     in.top_p = rp.top_p;
     in.S_ext = mass ? S_tot : 0ull;
     in.m_row = m; in.inv_T = pl.inv_T; in.u = src.u;
-    const bool inside = n <= kThreads ? select_small(in, sel, selq, sh, o) : select_and_draw(in, sel, selq, sh, o);
+    const bool inside = n <= kThreads ? select_small(in, sel, selq, sh, o) : select_large(in, sel, selq, reinterpret_cast<uint32_t*>(wl), sh, o);
     if (!inside && tid == 0) defer_row(A, sh, row, 7u);
 }
 

@@ -30,6 +30,9 @@ __global__ void __launch_bounds__(kThreads) merge_kernel(const __grid_constant__
     const int tid = threadIdx.x, b = blockIdx.x;
     uint64_t* sel = reinterpret_cast<uint64_t*>(smem);
     unsigned long long* selq = reinterpret_cast<unsigned long long*>(sel + kSelCap);
+    // (starts while the launch that writes the records may still be working)
+    grid_launch_dependents();
+    grid_dependency_wait();
     const float inv_T = __fdiv_rn(1.0f, A.temperature);
     const float c2 = inv_T * 1.44269504f;
     auto rec_of = [&](int g) { return A.gathered + (int64_t)g * A.seg_stride + (int64_t)b * A.row_stride; };
@@ -82,7 +85,7 @@ __global__ void __launch_bounds__(kThreads) merge_kernel(const __grid_constant__
     in.S_ext = 0;
     in.m_row = m; in.inv_T = inv_T; in.u = A.uniforms[b];
     if (n <= kThreads) select_small(in, sel, selq, sh, o);
-    else select_and_draw(in, sel, selq, sh, o);
+    else select_large(in, sel, selq, reinterpret_cast<uint32_t*>(selq + kSelCap), sh, o);
 }
 
 }  // namespace born

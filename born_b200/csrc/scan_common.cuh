@@ -31,11 +31,12 @@ constexpr int kMassBlock = 512;             // tokens per mass block of the whol
 constexpr int kSelCap = 1024;               // candidates the in-shared-memory selection handles
 constexpr int kHistBuckets = 128;           // the history list of a segment is grouped by block (or run of blocks)
 constexpr int kClusterMax = 8;              // slices of a row that exchange through distributed shared memory
-constexpr int kGrpList = 256;               // groups a warp lists before it reads them again
+constexpr int kGrpRound = 4096;             // group keys a CTA looks at before it reads the groups it found again
 constexpr int kBins = 1024;                 // bins of the finish's histograms
 constexpr uint32_t kDeadKey16 = 0x7Fu;      // group key of a group with nothing above -inf (-inf itself: 0x007FFFFF)
 // Shared memory of a finish: selection (rank keys, masses; before them the histograms) | group lists.
-constexpr int kWorkBytes = 2 * kSelCap * 8 + kScanWarps * kGrpList * 4;
+constexpr int kWorkBytes = 2 * kSelCap * 8 + kGrpRound * 2;
+static_assert(kGrpRound * 2 >= kBins * 8, "the larger selection keeps its bins where the group list was");
 // ... and of the exact search (fallback.cuh), which has the ring to itself
 constexpr int kExactBytes = 61440;
 
@@ -220,11 +221,12 @@ struct ScanShared {
     unsigned long long acc[4];
     float redf[kScanWarps];
     uint32_t redu[kScanWarps];
-    uint4 bcnt[kHistBuckets / 4];
+    uint4 bcnt[kHistBuckets / 4];   // counts of the history build; after it, the finish's map of candidates
     int nl, nw;
+    uint32_t ng[2], nh;             // groups listed (by parity of the round), history values added
     int found;
     unsigned long long before;
-    SearchScratch sc;
+    alignas(16) SearchScratch sc;
 };
 
 __device__ __forceinline__ float max3_nan(float a, float b, float c) {

@@ -169,6 +169,7 @@ __device__ __forceinline__ int hist_build(const ScanArgs& A, ScanShared& sh, uin
         list[offs[bk] + rank[r]] = ((unsigned long long)(mult[at[r]] + 1u) << 32) | tok;
     }
     cta_sync();
+    if (tid < kHistBuckets / 4) sh.bcnt[tid] = make_uint4(0u, 0u, 0u, 0u);  // (now the finish's map of candidates)
     return (int)n;
 }
 
@@ -385,7 +386,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) scan_kernel(const __grid_cons
         if (keys_smem && rank > 0) gk = cluster_map(gk, 0u);
         MassBlock* row_blocks = A.blocks + (int64_t)row * A.nblk;
         cta_sync();  // (the finish of the segment before is done with what the set-up writes)
-        if (tid == 0) sh.nl = 0;
+        if (tid == 0) { sh.nl = 0; sh.ng[0] = sh.ng[1] = sh.nh = 0; }
         int hn = 0, hs = 0;
         if constexpr (kHist) {
             if (!first_seg) hist_ids(A, q.b, ids);  // (those of the first row were fetched before the first copies)
