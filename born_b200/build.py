@@ -17,7 +17,7 @@ CSRC = os.path.join(HERE, "csrc")
 UNITS = ["capi.cu", "scan_f32.cu", "scan_f32_hist.cu", "scan_f32_mask.cu", "scan_f32_mask_hist.cu", "scan_bf16.cu", "scan_bf16_hist.cu",
          "scan_bf16_mask.cu", "scan_bf16_mask_hist.cu"]
 HEADERS = ["spec.cuh", "scan_common.cuh", "scan_kernel.cuh", "scan_inst.cuh", "scan_launch.cuh", "finish.cuh", "fallback.cuh",
-           "merge_kernel.cuh", "prepass.cuh", "spec_kernel.cuh", "warp_ring.cuh"]
+           "merge_kernel.cuh", "prepass.cuh", "spec_kernel.cuh", "warp_ring.cuh", "local_kernel.cuh"]
 DEPS = [os.path.join(CSRC, f) for f in UNITS + HEADERS]
 DEPS.append(os.path.join(ROOT, "include", "born_sampler.h"))
 OBJ_DIR = os.path.join(HERE, "build")

@@ -550,6 +550,32 @@ __device__ __forceinline__ void defer_row(const ScanArgs& A, ScanShared& sh, int
     if (A.slices == 0) A.deferred[row] = word;
 }
 
+// A key that at least k of the 256 keys a warp holds (eight per lane) reach, and not many more: by
+// bisection.  0 when fewer than k are alive.
+__device__ __forceinline__ uint32_t kth_of_maxima(const uint32_t (&v)[8], int k) {
+    auto reach = [&](uint32_t key) {
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) c += v[i] >= key ? 1 : 0;
+        return __reduce_add_sync(0xffffffffu, c);
+    };
+    uint32_t lo = kDeadKey16 + 1u;
+    if (reach(lo) < k) return 0u;
+    uint32_t hi = v[0], mn = v[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) { hi = max(hi, v[i]); mn = min(mn, v[i]); }
+    hi = __reduce_max_sync(0xffffffffu, hi) + 1u;
+    lo = max(lo, __reduce_min_sync(0xffffffffu, mn));
+    while (hi - lo > 1u) {  // k of the keys reach lo, fewer reach hi
+        const uint32_t mid = (lo + hi) >> 1;
+        const int c = reach(mid);
+        if (c >= k) lo = mid;
+        else hi = mid;
+        if (c >= k && c <= k + k / 16) break;
+    }
+    return lo;
+}
+
 // A key that at least k of the n 16-bit keys (key_of(i), zero: none) reach, and not many more.  Up to
 // half as many as there are threads: the k-th largest of the threads' own maxima -- k keys reach it, and
 // few more, since the k best seldom share a thread (50 of 4008 keys: 54 reach it).  Every warp holds all
@@ -577,29 +603,9 @@ __device__ __forceinline__ uint32_t kth_key(F key_of, int n, int k, float m, uin
         maxima[tid] = (uint16_t)mx;
         cta_sync();
         const uint4 w = reinterpret_cast<const uint4*>(maxima)[lane];
-        const uint32_t v[8] = {w.x & 0xFFFFu, w.x >> 16, w.y & 0xFFFFu, w.y >> 16, w.z & 0xFFFFu, w.z >> 16, w.w & 0xFFFFu, w.w >> 16};
-        auto reach = [&](uint32_t key) {
-            int c = 0;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) c += v[i] >= key ? 1 : 0;
-            return __reduce_add_sync(0xffffffffu, c);
-        };
-        uint32_t lo = kDeadKey16 + 1u;
-        if (reach(lo) >= k) {
-            uint32_t hi = v[0], mn = v[0];
-#pragma unroll
-            for (int i = 1; i < 8; ++i) { hi = max(hi, v[i]); mn = min(mn, v[i]); }
-            hi = __reduce_max_sync(0xffffffffu, hi) + 1u;
-            lo = max(lo, __reduce_min_sync(0xffffffffu, mn));
-            while (hi - lo > 1u) {  // k of the maxima reach lo, fewer reach hi
-                const uint32_t mid = (lo + hi) >> 1;
-                const int c = reach(mid);
-                if (c >= k) lo = mid;
-                else hi = mid;
-                if (c >= k && c <= k + k / 16) break;
-            }
-            return lo;
-        }
+        uint32_t v[8] = {w.x & 0xFFFFu, w.x >> 16, w.y & 0xFFFFu, w.y >> 16, w.z & 0xFFFFu, w.z >> 16, w.w & 0xFFFFu, w.w >> 16};
+        const uint32_t t = kth_of_maxima(v, k);
+        if (t) return t;
     }
     uint32_t mn = 0xFFFFu;
     auto see = [&](uint32_t key) { mn = min(mn, key > kDeadKey16 ? key : 0xFFFFu); };

@@ -36,28 +36,45 @@ __global__ void __launch_bounds__(kThreads) merge_kernel(const __grid_constant__
     const float inv_T = __fdiv_rn(1.0f, A.temperature);
     const float c2 = inv_T * 1.44269504f;
     auto rec_of = [&](int g) { return A.gathered + (int64_t)g * A.seg_stride + (int64_t)b * A.row_stride; };
-    // headers are read word by word: a record of an odd number of entries is only 8-byte aligned
-    float m = -INFINITY;
-    int inexact = 0;
-    for (int g = 0; g < A.G; ++g) {
-        const uint32_t* h = reinterpret_cast<const uint32_t*>(rec_of(g));
-        m = max_nan(m, __uint_as_float(__ldcg(h)));
-        inexact |= (int)(__ldcg(h + 3) & 2u);
-    }
-    float ls = 0.0f;
+    // Every warp folds the headers for itself, a lane per record (word by word: a record of an odd number
+    // of entries is only 8-byte aligned); then the warps share out the records' entries.  (A loop over the
+    // records with a read and an atomic each was a chain of G round trips to L2.)
+    const int lane = tid & 31, warp = tid >> 5;
+    float m = -INFINITY, ls = 0.0f;
+    int cnt = 0, inexact = 0;
     if (tid == 0) sh.nl = 0;
+    if (lane < A.G) {
+        const uint32_t* h = reinterpret_cast<const uint32_t*>(rec_of(lane));
+        m = __uint_as_float(__ldcg(h));
+        ls = __uint_as_float(__ldcg(h + 1));
+        cnt = (int)__ldcg(h + 2);
+        inexact = (int)(__ldcg(h + 3) & 2u);
+    }
     cta_sync();
-    for (int g = 0; g < A.G; ++g) {
-        const uint32_t* h = reinterpret_cast<const uint32_t*>(rec_of(g));
-        const float mg = __uint_as_float(__ldcg(h)), sg = __uint_as_float(__ldcg(h + 1));
-        if (sg > 0.0f) ls += sg * ex2_approx(__fmul_rn(mg - m, c2));
-        const int cnt = (int)__ldcg(h + 2);
+    const float mg = m;
+    m = warp_max_nan(m);
+    ls = ls > 0.0f ? ls * ex2_approx(__fmul_rn(mg - m, c2)) : 0.0f;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, d);
+    inexact = __any_sync(0xffffffffu, inexact);
+    for (int g = warp; g < A.G; g += kScanWarps) {
+        const int c = __shfl_sync(0xffffffffu, cnt, g);
         const unsigned long long* ent = reinterpret_cast<const unsigned long long*>(rec_of(g) + kRecordHdrBytes);
-        for (int i = tid; i < cnt; i += kThreads) {
-            const unsigned long long e = __ldcg(ent + i);
-            if (ck_alive(e)) {
-                const int pos = (int)smem_atom_add(&sh.nl, 1u);
-                if (pos < kSelCap) sel[pos] = e;
+        for (int i = 0; i < c; i += 64) {
+            unsigned long long e[2];
+            uint32_t ab[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) e[j] = i + 32 * j + lane < c ? __ldcg(ent + i + 32 * j + lane) : 0ull;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) ab[j] = __ballot_sync(0xffffffffu, ck_alive(e[j]));
+            int at = 0;
+            if (lane == 0) at = (int)smem_atom_add(&sh.nl, (uint32_t)(__popc(ab[0]) + __popc(ab[1])));
+            at = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int pos = at + __popc(ab[j] & ((1u << lane) - 1u));
+                if (ck_alive(e[j]) && pos < kSelCap) sel[pos] = e[j];
+                at += __popc(ab[j]);
             }
         }
     }

@@ -69,6 +69,7 @@ struct ScanSmem {
     int gkeys_cap;  // ... groups there is room for
     int list;       // history list, then the kHistBuckets + 1 bucket offsets
     int list_cap;
+    int per_warp;   // local_kernel: bytes of a warp's part (the offsets above are inside it)
     int total;
 };
 
@@ -204,6 +205,27 @@ inline ScanSmem scan_smem_layout(int elem_bytes, bool aligned, bool has_mask, in
     L.list = off;
     off += list;
     L.total = (off + 127) & ~127;
+    return L;
+}
+
+// local_kernel: a warp's part of the dynamic shared memory is ring | group keys | candidates | group list.
+constexpr int kLocalCap = 256;     // candidates (and listed groups) a warp has room for
+constexpr int kLocalMaxK = 128;    // top-k up to which the 256 maxima of a warp tell the k-th key well
+// (stages: 0 when the row is too long)
+inline ScanSmem local_smem_layout(int elem_bytes, int nb, int limit) {
+    ScanSmem L = {};
+    L.slot = ring_slot_bytes(elem_bytes, true);
+    const int fixed = nb * 64 + kLocalCap * 8 + kLocalCap * 2;
+    const int per = limit / kScanWarps / 128 * 128;
+    L.stages = per >= fixed + 2 * L.slot ? (per - fixed) / L.slot : 0;
+    if (L.stages > kScanStagesMax) L.stages = kScanStagesMax;
+    L.gkeys = L.stages * L.slot;
+    L.gkeys_cap = nb * 32;
+    L.work = L.gkeys + nb * 64;
+    L.list = L.work + kLocalCap * 8;
+    L.per_warp = (L.list + kLocalCap * 2 + 127) & ~127;
+    L.total = kScanWarps * L.per_warp;
+    if (L.total < kExactBytes) L.total = kExactBytes;
     return L;
 }
 

@@ -3,6 +3,7 @@
 //   SCAN_INST_T      the element type (float or uint16_t)
 //   SCAN_INST_MASK / SCAN_INST_HIST   whether the launches carry grammar masks / token histories
 //   SCAN_INST_ATTRS / SCAN_INST_LAUNCH   the names of the two functions of scan_launch.cuh
+//   SCAN_INST_LOCAL_ATTRS / SCAN_INST_LOCAL   (optional) local_kernel for the element type as well
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -12,6 +13,9 @@
 #include "scan_kernel.cuh"
 #include "fallback.cuh"
 #include "scan_launch.cuh"
+#ifdef SCAN_INST_LOCAL
+#include "local_kernel.cuh"
+#endif
 
 namespace born {
 namespace {
@@ -61,6 +65,18 @@ cudaError_t SCAN_INST_ATTRS() {
     if ((e = attr_one<true, 2>()) != cudaSuccess) return e;
     return attr_one<false, 1>();
 }
+
+#ifdef SCAN_INST_LOCAL
+cudaError_t SCAN_INST_LOCAL_ATTRS() {
+    return cudaFuncSetAttribute(local_kernel<SCAN_INST_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kScanSmemTwo);
+}
+cudaError_t SCAN_INST_LOCAL(const ScanArgs& A, int grid, cudaStream_t st) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[2];
+    scan_launch_config(A, grid, st, cfg, at);
+    return cudaLaunchKernelEx(&cfg, local_kernel<SCAN_INST_T>, A);
+}
+#endif
 
 #ifdef SCAN_INST_CLUSTERS
 // Clusters of `size` CTAs that the current device holds at once (any instantiation: they share the

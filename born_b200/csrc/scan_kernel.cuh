@@ -72,6 +72,15 @@ __device__ __forceinline__ void lse32(ThreadStats& st, const float (&v)[2][16], 
     st.s = __fadd2_rn(__fadd2_rn(s[0], s[1]), __fadd2_rn(s[2], s[3]));
 }
 
+// Maximum of a lane's group (NaN-propagating).
+__device__ __forceinline__ float group_max(const float (&v)[2][16]) {
+    float m8[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        m8[i] = max_nan(max3_nan(v[i >> 2][4 * (i & 3)], v[i >> 2][4 * (i & 3) + 1], v[i >> 2][4 * (i & 3) + 2]), v[i >> 2][4 * (i & 3) + 3]);
+    return max3_nan(max3_nan(m8[0], m8[1], m8[2]), max3_nan(m8[3], m8[4], m8[5]), max_nan(m8[6], m8[7]));
+}
+
 // ---- token history -----------------------------------------------------------------------------
 // Penalties touch at most BORN_MAX_HISTORY tokens of a row.  The global read of the ids is the only
 // memory round trip of the build; for a CTA's first row it leaves before the CTA's first copies
@@ -454,11 +463,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) scan_kernel(const __grid_cons
                     for (int i = 0; i < 16; ++i)
                         if (group_pos<T>(h, i, kAligned) >= left) v[h][i] = -INFINITY;
             }
-            float m8[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                m8[i] = max_nan(max3_nan(v[i >> 2][4 * (i & 3)], v[i >> 2][4 * (i & 3) + 1], v[i >> 2][4 * (i & 3) + 2]), v[i >> 2][4 * (i & 3) + 3]);
-            const float mt = max3_nan(max3_nan(m8[0], m8[1], m8[2]), max3_nan(m8[3], m8[4], m8[5]), max_nan(m8[6], m8[7]));
+            const float mt = group_max(v);
             st.mx = max_nan(st.mx, mt);
             if (!mass || pl.window) gk[j * 32 + lane] = (uint16_t)(zkey(mt) >> 16);
             if (want_lse) lse32(st, v, mt, pl.c2);

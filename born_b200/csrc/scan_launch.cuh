@@ -28,6 +28,11 @@ SCAN_UNIT(bf16_hist)
 SCAN_UNIT(bf16_mask)
 SCAN_UNIT(bf16_mask_hist)
 #undef SCAN_UNIT
+// local_kernel (a warp per virtual row): rows on 16-byte boundaries, no mask, no token history.
+cudaError_t local_attrs_f32();
+cudaError_t local_attrs_bf16();
+cudaError_t local_launch_f32(const ScanArgs& A, int grid, cudaStream_t st);
+cudaError_t local_launch_bf16(const ScanArgs& A, int grid, cudaStream_t st);
 // Clusters of `size` CTAs of the streaming kernel that the current device holds at once.
 cudaError_t scan_max_clusters(int size, int* count);
 

@@ -1,0 +1,95 @@
+"""The branches of a row's finish and the warp-per-row kernel, at the sizes where they change: tokens,
+statuses, kept lists and probabilities bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+from born_b200 import workloads as W
+from tests.test_gpu_parity import assert_parity, run_both
+
+pytestmark = pytest.mark.gpu
+
+
+def _logits(seed, B, V, dtype, scale=3.0):
+    z = (W.normal(seed, 11, B * V) * scale).astype(np.float32).reshape(B, V)
+    if dtype == "f32":
+        return z
+    return (z.view(np.uint32) >> 16).astype(np.uint16)  # (truncated: any bf16 values will do, ties included)
+
+
+# either side of 32, 64, 128, 256 candidates (threads per candidate, then the counting sort), of 128 (bisection
+# over thread maxima, then bins) and up to the candidate limit; top-p off and on
+@pytest.mark.parametrize("k", [1, 31, 32, 33, 64, 65, 128, 129, 255, 256, 257, 600, 1000])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_candidate_counts_either_side_of_every_split(sampler, oracle, k, dtype):
+    B, V = 6, 20011 if dtype == "f32" else 20008
+    z, u = _logits(k, B, V, dtype), W.uniform_f32(k, 2, B)
+    for top_p in (0.0, 0.93):
+        got, ref = run_both(sampler, oracle, z, dict(temperature=4.0, top_k=k, top_p=top_p), u, want_kept=1024)
+        assert_parity(got, ref)
+
+
+# min-p and top-p alone leave their own numbers of candidates
+@pytest.mark.parametrize("params", [dict(temperature=3.0, min_p=0.02), dict(temperature=1.5, top_p=0.9),
+                                    dict(temperature=2.0, min_p=0.005, top_p=0.97)])
+def test_candidate_counts_of_rows_without_top_k(sampler, oracle, params):
+    B, V = 12, 32000
+    z = _logits(5, B, V, "f32") * np.linspace(0.6, 1.6, B, dtype=np.float32)[:, None]
+    got, ref = run_both(sampler, oracle, z, params, W.uniform_f32(5, 2, B), want_kept=1024)
+    assert_parity(got, ref)
+
+
+# every live group belongs to one thread: its maxima cannot tell the k-th key
+def test_fewer_live_maxima_than_top_k(sampler, oracle):
+    B, V = 3, 131072
+    z = _logits(9, B, V, "f32")
+    live = (np.arange(V) // 32) % 256 == 7
+    mask = np.packbits(np.tile(live, (B, 1)), axis=1, bitorder="little").view(np.uint32)
+    got, ref = run_both(sampler, oracle, z, dict(temperature=1.0, top_k=50), W.uniform_f32(9, 2, B), mask=mask)
+    assert_parity(got, ref)
+
+
+# history tokens among the candidates, beside them, and such as share a bit of the 4096-bit map with one
+@pytest.mark.parametrize("B", [2, 40])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_history_tokens_among_the_candidates(sampler, oracle, B, dtype):
+    V, H = 50176, 300
+    z = _logits(3, B, V, dtype)
+    val = z if dtype == "f32" else (z.astype(np.uint32) << 16).view(np.float32)
+    order = np.argsort(-val, axis=1)
+    hist = np.empty((B, H), np.int32)
+    hist[:, :60] = order[:, :120:2]
+    hist[:, 60:120] = (order[:, 1:121:2] + 4096) % V
+    hist[:, 120:] = W.randint(3, 4, B * (H - 120), V).reshape(B, -1)
+    for params in (dict(temperature=0.9, top_k=50, top_p=0.95, repetition_penalty=1.2),
+                   dict(temperature=0.9, min_p=0.05, top_p=0.9, frequency_penalty=0.5, presence_penalty=-0.4),
+                   dict(temperature=0.0, frequency_penalty=0.7)):
+        got, ref = run_both(sampler, oracle, z, params, W.uniform_f32(3, 2, B), hist=hist)
+        assert_parity(got, ref)
+
+
+# a warp per row: one block, a block and a granule, ragged tails, the largest top-k; and the rows that leave
+# its path: equal values beyond its candidate list, nothing alive, NaN and infinity
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("V,G,k", [(520, 8, 8), (1024, 8, 16), (1032, 8, 16), (8200, 8, 64), (9216, 8, 128), (9016, 4, 1)])
+def test_warp_per_row_segments(sampler, oracle, V, G, k, dtype):
+    B = 320 // G + 8
+    z = _logits(V + k, B, V * G, dtype)
+    ninf, pinf, nan, one = ((np.float32(x) for x in (-np.inf, np.inf, np.nan, 1.0)) if dtype == "f32" else
+                            (np.uint16(x) for x in (0xFF80, 0x7F80, 0x7FC0, 0x3F80)))
+    z[0] = ninf
+    z[1, V:2 * V] = one        # one segment all equal
+    z[2, V * G - 1] = nan
+    z[3, 5] = pinf
+    z[4, 7:] = ninf            # fewer tokens than top-k
+    z[5] = ninf
+    z[5, V * G - 3:] = one
+    got, ref = run_both(sampler, oracle, z, dict(temperature=1.3, top_k=k, top_p=0.95), W.uniform_f32(V, 2, B), segments=G,
+                        want_kept=min(1024, k * G))
+    assert_parity(got, ref)
+    # (the oracle's own log-sum-exp adds in fp32 one term after another: float64 is the measure)
+    val = z if dtype == "f32" else (z.astype(np.uint32) << 16).view(np.float32)
+    for b in np.nonzero(ref["status"] == 0)[0]:
+        x = val[b].astype(np.float64) / float(np.float32(1.3))
+        truth = x.max() + np.log(np.exp(x - x.max()).sum())
+        # 1e-5 relative on sum(exp) is 1e-5 absolute on its logarithm
+        assert abs(got["lse"][b] - truth) <= 1e-5 + 1e-6 * abs(truth), (b, got["lse"][b], truth)
