@@ -219,21 +219,20 @@ int launch_scan(Handle* h, const ScanArgs& A, int dtype, bool aligned, int grid,
 
 // First half of vocab-sharded sampling: the k best of every virtual row.
 int launch_local(Handle* h, ScanArgs& A, int dtype, bool aligned, int grid, cudaStream_t st) {
-    // A warp per row once rows would have to queue for a CTA, if they are short for their number: a warp
-    // needs some 1.5 us per block of 1024 tokens, whatever the others do.  Segments of 32 blocks (bf16, top-k
-    // 64, with the merge): 512 rows 53.8 us against 46.2 with a CTA per row, 1024 rows 54.9 against 68.7,
-    // 4096 rows 104 against 181; of 8 blocks: 512 rows 33 against 41.  Its 256 maxima must tell the k-th key.
+    // A warp per row once a CTA per row would take more than two waves and a half.  The warps stay busy
+    // for one row's time however few rows there are: bf16 segments of 32000, top-k 50, with the merge, 512
+    // rows take 42.7 us against 30.2 in waves of CTAs, 696 rows 42.3 against 39.4, 1024 rows 43.1 against
+    // 52.4, 2048 rows 53.7 against 88.4; segments of 16384 cross at 690 rows, fp32 ones of 32000 at 700.
+    // The 256 maxima of a warp must tell the k-th key.
     const int64_t rows = (int64_t)A.B * A.G;
-    if (aligned && !A.mask && !A.history && !A.row_params && rows > h->max_grid && rows >= 32 * (int64_t)A.nb && A.params.top_k <= kLocalMaxK &&
+    if (aligned && !A.mask && !A.history && !A.row_params && 2 * rows >= 5 * (int64_t)h->max_grid && A.params.top_k <= kLocalMaxK &&
         (A.V + kGrpTok - 1) / kGrpTok >= 2 * A.params.top_k) {
         const ScanSmem L = local_smem_layout(dtype == BORN_DTYPE_F32 ? 4 : 2, A.nb, kScanSmemTwo);
         if (L.stages >= 2) {
             A.L = L;
             A.slices = 0;
             A.cluster = 0;
-            const int64_t need = (rows + kScanWarps - 1) / kScanWarps;
-            const int g = need < h->max_grid ? (int)need : h->max_grid;
-            const cudaError_t e = dtype == BORN_DTYPE_F32 ? local_launch_f32(A, g, st) : local_launch_bf16(A, g, st);
+            const cudaError_t e = dtype == BORN_DTYPE_F32 ? local_launch_f32(A, h->max_grid, st) : local_launch_bf16(A, h->max_grid, st);
             if (e != cudaSuccess) return fail(h, BORN_ERR_CUDA, "local kernel launch failed: %s", cudaGetErrorString(e));
             h->launches++;
             return BORN_OK;
@@ -304,7 +303,15 @@ int fill_scan(Handle* h, ScanArgs& A, int B, int G, int V, int dtype, const void
         if (!A.cluster && s > 1 && rows * s > h->rec_slots) s = h->rec_slots / rows;
         A.slices = s > 1 ? (int)s : 1;
         *grid = (int)rows * A.slices;
+    } else if (A.nb <= 48 || 4 * rows >= 5 * (int64_t)h->max_grid) {
+        // One CTA per row, in waves.  Its keys and history stay in its shared memory and its finish
+        // overlaps the next row's stream in the SM's other CTA, where a range that ends in mid-row pays
+        // for records, a ticket and a finish out of L2.  Top-k 50, fp32, ranges -> waves: 400 rows of 32768
+        // 30.1 -> 24.5 us, 512 of 131072 59.6 -> 55.4; 380 bf16 segments of 39360 60 -> 47.
+        A.slices = 1;
+        *grid = (int)rows;
     } else {
+        // long rows, and a second wave that would be nearly empty (300 of 131072: 39.5 us, in waves 45.6)
         A.slices = 0;
         *grid = h->max_grid;
     }

@@ -13,11 +13,6 @@
 namespace born {
 
 constexpr int kThreads = 256;        // threads per CTA in the row kernels
-constexpr int kTileBytes = 16384;    // bytes of logits per pipeline stage (4096 fp32 / 8192 bf16)
-constexpr int kStages = 5;           // bulk-copy stages in flight per CTA
-constexpr int kMaxK = 1024;          // BORN_MAX_TOP_K / BORN_MAX_CANDIDATES
-constexpr int kCandCap = 2048;       // candidate buffer entries (>= kMaxK + one half piece)
-constexpr int kHistCap = 1024;       // history ids held per CTA
 constexpr uint32_t kIdxMask = 0xFFFFFFu;
 constexpr int kRecordHdrBytes = 32;
 
@@ -140,36 +135,18 @@ __device__ __forceinline__ void smem_red_add(void* p, uint32_t v) {
 __device__ __forceinline__ void smem_red_or(void* p, uint32_t v) {
     asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
 }
-__device__ __forceinline__ void smem_red_max(void* p, uint32_t v) {
-    asm volatile("red.shared.max.u32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
-}
-__device__ __forceinline__ void smem_red_min(void* p, uint32_t v) {
-    asm volatile("red.shared.min.u32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
-}
-
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
 __device__ __forceinline__ void mbar_fence_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void fence_proxy_async() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
-// Non-multicast bulk copy global -> this CTA's shared memory; both addresses 16-byte
-// aligned, bytes a multiple of 16.
-__device__ __forceinline__ void bulk_load(void* dst_smem, const void* src_gmem, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst_smem)),
-                 "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-// Bounded wait: gives up after about two seconds of wall-clock time (or kMbarSpinLimit
-// probes, whichever comes first) and reports false; the caller records the failure and
-// leaves the kernel in an orderly way.
+// Limits of a wait (warp_ring.cuh): about two seconds of wall-clock time or kMbarSpinLimit
+// probes, whichever comes first; the caller records the failure and leaves the kernel in an
+// orderly way.
 constexpr uint32_t kMbarSpinLimit = 1u << 26;
 constexpr unsigned long long kMbarTimeoutNs = 2000000000ull;
 __device__ __forceinline__ unsigned long long global_timer_ns() {
@@ -177,32 +154,8 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    const uint32_t addr = smem_u32(bar);
-    unsigned long long t0 = 0;
-    for (uint32_t it = 0; it < kMbarSpinLimit; ++it) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(addr), "r"(parity)
-            : "memory");
-        if (ok) return true;
-        if ((it & 63u) == 63u) {
-            const unsigned long long now = global_timer_ns();
-            if (t0 == 0) t0 = now;
-            else if (now - t0 > kMbarTimeoutNs) return false;
-        }
-    }
-    return false;
-}
-
 // ---- barriers of the 256 compute threads ----------------------------------------------------
-// The row kernels run 256 compute threads plus, in the streaming kernel, one producer warp
-// that only issues bulk copies.  Everything the compute threads synchronise on uses named
-// barrier 1 with a count of 256, so the producer warp never takes part.
+// Named barrier 1 with a count of 256.
 __device__ __forceinline__ void cta_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 __device__ __forceinline__ int cta_sync_or(int pred) {
     int r;
@@ -227,70 +180,6 @@ __device__ __forceinline__ int cta_sync_count(int pred) {
         : "memory");
     return r;
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// Bounded wait that also gives up when *abort becomes non-zero (set by the compute threads
-// when they leave early).
-__device__ __forceinline__ bool mbar_wait_or_abort(uint64_t* bar, uint32_t parity, const volatile int* abort) {
-    const uint32_t addr = smem_u32(bar);
-    unsigned long long t0 = 0;
-    for (uint32_t it = 0; it < kMbarSpinLimit; ++it) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(addr), "r"(parity)
-            : "memory");
-        if (ok) return true;
-        if (*abort) return false;
-        if ((it & 63u) == 63u) {
-            const unsigned long long now = global_timer_ns();
-            if (t0 == 0) t0 = now;
-            else if (now - t0 > kMbarTimeoutNs) return false;
-        }
-    }
-    return false;
-}
-
-// Bounded wait that returns 1 when the phase completed, 2 as soon as *event is non-zero
-// (checked between probes by the whole warp, so the answer is warp-uniform), 0 on a timeout.
-__device__ __forceinline__ int mbar_wait_or_event(uint64_t* bar, uint32_t parity, const volatile int* event) {
-    const uint32_t addr = smem_u32(bar);
-    {   // the tile is usually there already: one probe, no votes
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(addr), "r"(parity)
-            : "memory");
-        if (ok) return 1;
-    }
-    unsigned long long t0 = 0;
-    for (uint32_t it = 0; it < kMbarSpinLimit; ++it) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(addr), "r"(parity)
-            : "memory");
-        if (__all_sync(0xffffffffu, ok != 0)) return 1;
-        if (__any_sync(0xffffffffu, *event != 0)) return 2;
-        if ((it & 63u) == 63u) {
-            const unsigned long long now = global_timer_ns();
-            if (t0 == 0) t0 = now;
-            else if (__any_sync(0xffffffffu, now - t0 > kMbarTimeoutNs)) return 0;
-        }
-    }
-    return 0;
-}
-
 // ---- warp helpers ------------------------------------------------------------------------
 __device__ __forceinline__ uint64_t shfl_u64(uint64_t v, int src) {
     uint32_t lo = __shfl_sync(0xffffffffu, (uint32_t)v, src);

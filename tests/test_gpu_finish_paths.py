@@ -67,12 +67,24 @@ def test_history_tokens_among_the_candidates(sampler, oracle, B, dtype):
         assert_parity(got, ref)
 
 
+# more rows than CTAs fit at once: a CTA per row in waves, and ranges for long rows with a nearly empty second wave
+@pytest.mark.parametrize("B,V,dtype", [(297, 1000, "f32"), (301, 50176, "f32"), (303, 50001, "bf16"), (375, 50176, "bf16"), (600, 1031, "bf16")])
+def test_more_rows_than_fit_at_once(sampler, oracle, B, V, dtype):
+    z, u = _logits(B, B, V, dtype), W.uniform_f32(B, 2, B)
+    hist = W.randint(B, 3, B * 40, V).astype(np.int32).reshape(B, 40)
+    for params in (dict(temperature=0.8, top_k=40, top_p=0.9, repetition_penalty=1.3), dict(temperature=0.0)):
+        got, ref = run_both(sampler, oracle, z, params, u, hist=hist)
+        assert_parity(got, ref)
+    got, ref = run_both(sampler, oracle, z, dict(temperature=0.7, top_p=0.8), u)
+    assert_parity(got, ref, check_kept=False)
+
+
 # a warp per row: one block, a block and a granule, ragged tails, the largest top-k; and the rows that leave
 # its path: equal values beyond its candidate list, nothing alive, NaN and infinity
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("V,G,k", [(520, 8, 8), (1024, 8, 16), (1032, 8, 16), (8200, 8, 64), (9216, 8, 128), (9016, 4, 1)])
 def test_warp_per_row_segments(sampler, oracle, V, G, k, dtype):
-    B = 320 // G + 8
+    B = 752 // G
     z = _logits(V + k, B, V * G, dtype)
     ninf, pinf, nan, one = ((np.float32(x) for x in (-np.inf, np.inf, np.nan, 1.0)) if dtype == "f32" else
                             (np.uint16(x) for x in (0xFF80, 0x7F80, 0x7FC0, 0x3F80)))
