@@ -48,11 +48,14 @@ struct SelectIn {
     float m_row, inv_T, u;
 };
 
-// Threads that share the loops over one of n <= kThreads candidates: log2.  The loops are chains of
+// Threads that share the loops over one of n candidates: log2.  The loops are chains of
 // shared-memory reads, so the CTA's 256 threads are dealt over (candidate, part of the loop).
 __device__ __forceinline__ int split_lg(int n) { return n <= 32 ? 3 : n <= 64 ? 2 : n <= 128 ? 1 : 0; }
+// Candidates up to which every one is compared with every other (select_small).  The comparisons are quadratic:
+// 200 candidates took 13.4 us of a merge launch that sorts 400 in 9.9.
+constexpr int kSmallMax = 128;
 
-// Selection and draw over n <= kThreads candidates in shared memory (sel: rank keys; selq: scratch for
+// Selection and draw over n <= kSmallMax candidates in shared memory (sel: rank keys; selq: scratch for
 // their masses and, from kThreads on, for the masses of the kept ones).  Nothing is sorted: one loop over
 // the candidates gives each its rank (the number of larger keys: keys are unique, the token index is
 // part of them) and the mass ahead of it, and since a mass never grows along the rank order the kept
@@ -195,7 +198,7 @@ __device__ __forceinline__ int find_bin(F total_of, unsigned long long target, u
     return sh.found;
 }
 
-// Selection and draw over kThreads < n <= kSelCap candidates, the same rules, four candidates per thread.
+// Selection and draw over kSmallMax < n <= kSelCap candidates, the same rules, four candidates per thread.
 // A counting sort puts them in rank order: bins of equal width in value from the best candidate down,
 // places inside a bin by comparison.  Then the masses are scanned in rank order, and the draw finds its
 // token through bins of the token index.  (Three radix descents, over keys, masses and indices, took
@@ -1063,7 +1066,7 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
     in.top_p = rp.top_p;
     in.S_ext = mass ? S_tot : 0ull;
     in.m_row = m; in.inv_T = pl.inv_T; in.u = src.u;
-    const bool inside = n <= kThreads ? select_small(in, sel, selq, sh, o) : select_large(in, sel, selq, reinterpret_cast<uint32_t*>(wl), sh, o);
+    const bool inside = n <= kSmallMax ? select_small(in, sel, selq, sh, o) : select_large(in, sel, selq, reinterpret_cast<uint32_t*>(wl), sh, o);
     if (!inside && tid == 0) defer_row(A, sh, row, 7u);
 }
 

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kThreads) merge_kernel(const __grid_constant__
     in.top_p = A.top_p;
     in.S_ext = 0;
     in.m_row = m; in.inv_T = inv_T; in.u = A.uniforms[b];
-    if (n <= kThreads) select_small(in, sel, selq, sh, o);
+    if (n <= kSmallMax) select_small(in, sel, selq, sh, o);
     else select_large(in, sel, selq, reinterpret_cast<uint32_t*>(selq + kSelCap), sh, o);
 }
 
