@@ -4,9 +4,10 @@
 // Work decomposition.  A row is cut into blocks of 1024 tokens, counted from its first token.  The
 // part of a row inside one CTA is a *segment*; its blocks are dealt to the CTA's eight warps, each
 // of which streams its own (warp_ring.cuh).  While the rows fit the GPU (rows <= two CTAs per SM)
-// every row is given `slices` CTAs of its own, each with one segment; beyond that the blocks of
-// all rows form one sequence that is cut into equal contiguous ranges, one per CTA, so that a CTA
-// may end in mid-row.  A row that one CTA streamed from first to last block is finished by it
+// every row is given `slices` CTAs of its own, each with one segment; more rows take a CTA each, in
+// waves.  Only long rows with a nearly empty second wave form one sequence of blocks that is cut
+// into equal contiguous ranges, one per CTA, so that a CTA may end in mid-row (fill_scan in capi.cu
+// has the rule).  A row that one CTA streamed from first to last block is finished by it
 // at once.  The slices of a row, up to eight, form a thread-block cluster: they write their keys,
 // history values and statistics straight into the first one's shared memory, which finishes the row
 // after one cluster barrier.  Otherwise (more slices, or ranges) the segments leave records in scratch
