@@ -664,8 +664,20 @@ __device__ __forceinline__ uint32_t kth_key(F key_of, int n, int k, float m, uin
     const int b = sh.found;
     if (b < 0) return kDeadKey16 + 1u;
     if (b == kBins - 1 || scale == 0.0f) return lo;
-    // the lowest key of bin b (a key lower: the bins' own rounding)
-    return max((zkey(m - __fdiv_rn((float)(b + 1), scale)) >> 16) - 1u, lo);
+    // The smallest key that was counted into the bins up to b: k keys reach it by that count.  (An edge
+    // worked back from the bin's number would carry the rounding of m - z, half a unit in the last place of
+    // m, which is many steps of a key that is small beside m.)
+    uint32_t low = 0xFFFFu;
+    auto counted = [&](uint32_t key) { low = key >= lo && bin_of(key) <= b ? min(low, key) : low; };
+#pragma unroll
+    for (int i = 0; i < kReg; ++i) counted(kk[i]);
+    for (int g = tid + kReg * kThreads; g < n; g += kThreads) counted(key_of(g));
+    low = __reduce_min_sync(0xffffffffu, low);
+    if (lane == 0) sh.redu[warp] = low;
+    cta_sync();
+#pragma unroll
+    for (int w = 0; w < kScanWarps; ++w) low = min(low, sh.redu[w]);
+    return low;
 }
 
 // Raw logit of token `tok` of the row at `base` (no mask, no penalties).

@@ -48,6 +48,40 @@ def test_fewer_live_maxima_than_top_k(sampler, oracle):
     assert_parity(got, ref)
 
 
+# top-k above 128 (bins over the keys) where the k-th value is tiny beside the maximum: one unit in the last
+# place of the maximum spans many steps of its key.  Rows of one value beside one outlier (all ties: the exact
+# search) and of small normal values
+@pytest.mark.parametrize("k", [100, 150, 200, 600])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("segments", [1, 4])
+def test_kth_value_tiny_beside_the_maximum(sampler, oracle, k, dtype, segments):
+    if segments > 1 and k > 256:
+        pytest.skip("a segment's top-k is limited to 256")
+    V, outlier = 32768, [17.0, 40.0, 11.0, 21.5, 20.5, 48.7, 50.2]
+    z = (W.normal(30, 1, len(outlier) * V) * 1e-6).astype(np.float32).reshape(-1, V)
+    for b, v in enumerate([1e-6, 1e-5, -1e-5, 1e-6, 3e-5]):
+        z[b] = v
+    z[:, 3] = outlier
+    logits = z if dtype == "f32" else W.f32_to_bf16_bits(z).reshape(z.shape)
+    u = W.uniform_f32(30, 2, len(outlier))
+    for params in (dict(temperature=4.0, top_k=k), dict(temperature=4.0, top_k=k, top_p=0.999)):
+        got, ref = run_both(sampler, oracle, logits, params, u, segments=segments, want_kept=1024)
+        assert_parity(got, ref)
+
+
+# ... and the way a smaller top-k gets there: a mask leaves all live groups to one thread
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_kth_value_tiny_beside_the_maximum_with_few_live_maxima(sampler, oracle, dtype):
+    B, V, k = 3, 131072, 10
+    z = (W.normal(31, 1, B * V) * 1e-6).astype(np.float32).reshape(B, V)
+    live = (np.arange(V) // 32) % 256 == 7
+    z[:, 7 * 32] = [48.7, 17.0, 21.5]
+    mask = np.packbits(np.tile(live, (B, 1)), axis=1, bitorder="little").view(np.uint32)
+    logits = z if dtype == "f32" else W.f32_to_bf16_bits(z).reshape(z.shape)
+    got, ref = run_both(sampler, oracle, logits, dict(temperature=4.0, top_k=k), W.uniform_f32(31, 2, B), mask=mask)
+    assert_parity(got, ref)
+
+
 # history tokens among the candidates, beside them, and such as share a bit of the 4096-bit map with one
 @pytest.mark.parametrize("B", [2, 40])
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
