@@ -53,7 +53,7 @@ __device__ __forceinline__ void fb_history(FbCtx& c) {
     len = max(0, min(min(len, A.history_stride), BORN_MAX_HISTORY));
     const int32_t* gh = A.history + (int64_t)c.b * A.history_stride;
     for (int p = tid; p < len; p += kThreads) {
-        const long long tok = (long long)__ldg(gh + p) - (long long)c.g * c.V;
+        const long long tok = (long long)__ldcg(gh + p) - (long long)c.g * c.V;  // (hist_ids: not read-only)
         if (tok < 0 || tok >= c.V) continue;
         uint32_t slot = ((uint32_t)tok * 2654435761u) >> 21;
         for (int probe = 0; probe < kFbHash; ++probe) {

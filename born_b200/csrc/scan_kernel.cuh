@@ -88,15 +88,17 @@ __device__ __forceinline__ float group_max(const float (&v)[2][16]) {
 constexpr int kHistPer = BORN_MAX_HISTORY / kThreads;  // history ids per thread
 
 __device__ __forceinline__ void hist_ids(const ScanArgs& A, int b, int (&ids)[kHistPer]) {
-    // the ids do not wait for the length: both reads leave together, the length cuts afterwards
+    // the ids do not wait for the length: both reads leave together, the length cuts afterwards.  (Not
+    // through the read-only path: the launch before this one, which may still have been running when this
+    // one began, appends to the ring that the generate loop passes here.)
     const int cap = min(A.history_stride, (int)BORN_MAX_HISTORY);
     const int32_t* gh = A.history + (int64_t)b * A.history_stride;
 #pragma unroll
     for (int r = 0; r < kHistPer; ++r) {
         const int p = (int)threadIdx.x + r * kThreads;
-        ids[r] = p < cap ? __ldg(gh + p) : -1;
+        ids[r] = p < cap ? __ldcg(gh + p) : -1;
     }
-    const int len = A.history_len ? __ldg(A.history_len + b) : cap;
+    const int len = A.history_len ? __ldcg(A.history_len + b) : cap;
 #pragma unroll
     for (int r = 0; r < kHistPer; ++r)
         if ((int)threadIdx.x + r * kThreads >= len) ids[r] = -1;

@@ -172,3 +172,42 @@ def test_device_history_with_one_cta_per_row(sampler, oracle, cap, top_k):
     assert np.array_equal(fin.astype(bool), finished)
     for b in range(B):
         assert total[b] == len(hist[b])
+
+
+@pytest.mark.parametrize("B,dtype,top_k", [(1, "f32", 6), (8, "bf16", 6), (64, "f32", 6), (300, "f32", 6), (8, "f32", 0)],
+                         ids=["one-row", "bf16", "cluster-and-alone", "waves", "whole-row-draw"])
+def test_steps_queued_back_to_back_see_each_other_s_tokens(oracle, B, dtype, top_k):
+    # every step is in the stream before the first one starts, so that each launch begins while the one
+    # before it, which appends to the ring it reads, still runs; the strong penalties make a step's
+    # distribution depend on the token of the step before
+    import torch
+    from born_b200 import Sampler, SamplingConfig
+    V, cap, steps, P = 33000, 24, 40, 4
+    params = dict(temperature=0.7, top_k=top_k, repetition_penalty=1.5, frequency_penalty=1.0, presence_penalty=0.5)
+    cfg, op = SamplingConfig(**params), oracle.make_params(**params)
+    z = (W.normal(700 + B, 1, B * V) * 2.0).astype(np.float32).reshape(B, V)
+    z[:, 100:108] += 12.0
+    logits = W.f32_to_bf16_bits(z).reshape(B, V) if dtype == "bf16" else z
+    ld = torch.from_numpy(logits.view(np.int16).copy()).cuda().view(torch.bfloat16) if dtype == "bf16" else _dev(logits)
+    prompts = W.randint(700, 2, B * P, V).astype(np.int32).reshape(B, P)
+    us = [W.uniform_f32(700 + t, 3, B) for t in range(steps)]
+    s = Sampler(device=0, max_batch=B, max_vocab=V)
+    try:
+        s.history_create(cap)
+        s.history_reset(_dev(prompts))
+        ud = [_dev(u) for u in us]
+        s.sample(ld, uniforms=ud[0], config=cfg)  # (whatever is set up on a first call)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(50_000_000)  # some 25 ms: the host is through with the loop before the first step runs
+        outs = [s.sample_next(ld, uniforms=u, config=cfg) for u in ud]
+        torch.cuda.synchronize()
+        hist = prompts
+        for t in range(steps):
+            tail = np.ascontiguousarray(hist[:, -cap:])
+            ref = oracle.sample(logits, op, uniforms=us[t], history=tail, want_kept=1, nthreads=8)
+            tok = outs[t]["token"].cpu().numpy()
+            assert np.array_equal(tok, ref["token"]), (t, np.nonzero(tok != ref["token"])[0][:8])
+            assert np.array_equal(outs[t]["status"].cpu().numpy(), ref["status"]), t
+            hist = np.concatenate([hist, tok[:, None]], axis=1)
+    finally:
+        s.close()
