@@ -931,31 +931,104 @@ int32_t born_mask_wait(void* handle, void* stream) {
     return BORN_OK;
 }
 
+// The launches of born_debug_expire_wait: geometry, the block whose copy is withheld, and the caller rows
+// that have to report the failure (bit b; the others finish).
+namespace {
+struct ExpireCase {
+    int rows, G, blocks;   // caller rows, vocabulary segments, blocks per virtual row
+    int slices;            // 0: contiguous ranges over `grid` CTAs
+    int cluster, grid;
+    int local;             // 0: sampling; 1: records and merge, scan_kernel; 2: records and merge, local_kernel
+    int skip;
+    uint32_t failing;
+    int ties;              // all logits equal
+};
+constexpr ExpireCase kExpireCases[] = {
+    {1, 1, 12, 1, 0, 1, 0, 5, 0x1u, 0},    // a CTA that has its row to itself
+    {1, 1, 48, 3, 1, 3, 0, 5, 0x1u, 0},    // the first CTA of a cluster, which finishes the row
+    {1, 1, 48, 3, 1, 3, 0, 40, 0x1u, 0},   // ... another one
+    {1, 1, 48, 3, 0, 3, 0, 20, 0x1u, 0},   // slices that exchange through records and a ticket
+    {3, 1, 16, 0, 0, 2, 0, 30, 0x6u, 0},   // ranges: the second CTA, in the middle of the second row
+    {3, 1, 16, 0, 0, 2, 1, 30, 0x6u, 0},   // ... records
+    {4, 4, 2, 0, 0, 1, 2, 11, 0xAu, 0},    // a warp per row: one warp, with virtual rows 5 and 13
+    {4, 4, 2, 0, 0, 1, 2, 11, 0xFu, 1},    // ... the other warps' rows wait for the exact search
+};
+
+int expire_one(Handle* h, const ExpireCase& c, uint8_t* buf, float* host, cudaStream_t st) {
+    const int V = c.blocks * kBlkTok, K = 4;
+    const size_t n = (size_t)c.rows * c.G * V;
+    for (size_t i = 0; i < n; ++i) host[i] = c.ties ? 0.0f : (float)((uint32_t)i * 2654435761u >> 8);
+    uint8_t* out = buf + n * 4;  // statuses, tokens, uniforms (16 each), packed records
+    CUDA_TRY(h, cudaMemcpyAsync(buf, host, n * 4, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(h, cudaMemsetAsync(out, 0, 3 * 64, st));
+    ScanArgs A;
+    memset(&A, 0, sizeof A);
+    int grid = 0, rc;
+    if ((rc = fill_scan(h, A, c.rows, c.G, V, BORN_DTYPE_F32, buf, (int64_t)c.G * V, nullptr, 0, 0, &grid))) return rc;
+    if (c.cluster && h->max_clusters[c.slices] < 1) return BORN_ERR_DEVICE_TIMEOUT;  // (no clusters to test)
+    A.slices = c.slices;
+    A.cluster = c.cluster;
+    A.L = c.local == 2 ? local_smem_layout(4, A.nb, kScanSmemTwo)
+                       : scan_smem_layout(4, true, false, 0, c.slices > 0, c.slices > 1 && !c.cluster ? 0 : A.nb * 32, kScanSmemTwo);
+    A.out_status = (int32_t*)out;
+    A.out_token = (int32_t*)(out + 64);
+    A.timeout_ns = 1000000ull;
+    A.debug_skip_blk = c.skip;
+    const int64_t rec = kRecordHdrBytes + 8 * K;
+    if (c.local) {
+        A.mode = kScanLocal;
+        A.params.temperature = 1.0f;
+        A.params.top_k = K;
+        A.packed = out + 3 * 64;
+        A.packed_row_stride = rec;
+        A.packed_seg_stride = rec * c.rows;
+    } else {
+        A.mode = kScanFull;
+        A.params.flags = BORN_FLAG_GREEDY;
+    }
+    if (c.local == 2) {
+        CUDA_TRY(h, local_launch_f32(A, c.grid, st));
+        h->launches++;
+    } else if ((rc = launch_scan(h, A, BORN_DTYPE_F32, true, c.grid, st))) {
+        return rc;
+    }
+    if (c.local) {
+        MergeArgs M;
+        memset(&M, 0, sizeof M);
+        M.gathered = A.packed; M.row_stride = rec; M.seg_stride = rec * c.rows;
+        M.B = c.rows; M.G = c.G;
+        M.temperature = 1.0f;
+        M.uniforms = (const float*)(out + 2 * 64);
+        M.out_token = A.out_token; M.out_status = A.out_status;
+        if ((rc = launch_merge(h, M, st))) return rc;
+    }
+    int32_t status[16];
+    CUDA_TRY(h, cudaMemcpyAsync(status, A.out_status, sizeof(int32_t) * c.rows, cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(h, cudaStreamSynchronize(st));
+    if ((rc = check_device_error(h)) != BORN_ERR_DEVICE_TIMEOUT) return rc;
+    for (int b = 0; b < c.rows; ++b) {
+        const int want = (c.failing >> b) & 1u ? 100 + BORN_ERR_DEVICE_TIMEOUT : BORN_ROW_OK;
+        if (status[b] != want)
+            return fail(h, BORN_ERR_CUDA, "expired wait, case %d: row %d reports status %d, not %d", (int)(&c - kExpireCases), b, status[b], want);
+    }
+    return BORN_ERR_DEVICE_TIMEOUT;
+}
+}  // namespace
+
 int32_t born_debug_expire_wait(void* handle, void* stream) {
     Handle* h = (Handle*)handle;
     if (!h || h->is_static) return fail(nullptr, BORN_ERR_INVALID_ARGUMENT, "handle is NULL");
     int rc = use_device(h);
     if (rc) return rc;
-    cudaStream_t st = (cudaStream_t)stream;
-    // twelve blocks of zeros, one row, greedy; one block's copy is withheld
-    const int V = 12 * kBlkTok;
-    const size_t bytes = (size_t)V * 4 + 64;
+    const size_t floats = 48 * (size_t)kBlkTok, bytes = floats * 4 + 4096;
     if ((rc = stage_reserve(h, 15, bytes))) return rc;
-    uint8_t* buf = (uint8_t*)h->stage[15].p;
-    CUDA_TRY(h, cudaMemsetAsync(buf, 0, bytes, st));
-    ScanArgs A;
-    memset(&A, 0, sizeof A);
-    int grid = 0;
-    if ((rc = fill_scan(h, A, 1, 1, V, BORN_DTYPE_F32, buf, V, nullptr, 0, 0, &grid))) return rc;
-    A.params.flags = BORN_FLAG_GREEDY;
-    A.out_token = (int32_t*)(buf + (size_t)V * 4);
-    A.out_status = (int32_t*)(buf + (size_t)V * 4 + 16);
-    A.mode = kScanFull;
-    A.timeout_ns = 1000000ull;
-    A.debug_skip_blk = 5;
-    if ((rc = launch_scan(h, A, BORN_DTYPE_F32, true, grid, st))) return rc;
-    CUDA_TRY(h, cudaStreamSynchronize(st));
-    return check_device_error(h);
+    float* host = (float*)malloc(floats * 4);
+    if (!host) return fail(h, BORN_ERR_UNSUPPORTED, "out of host memory");
+    rc = BORN_ERR_DEVICE_TIMEOUT;
+    for (const ExpireCase& c : kExpireCases)
+        if ((rc = expire_one(h, c, (uint8_t*)h->stage[15].p, host, (cudaStream_t)stream)) != BORN_ERR_DEVICE_TIMEOUT) break;
+    free(host);
+    return rc;
 }
 
 int32_t born_debug_exp(const float* x, float* y, int64_t n, void* stream) {

@@ -19,7 +19,7 @@ struct PackedHdr {  // 32 bytes: header of a packed shard / segment record (the 
     float m;        // maximum of the shard's row (NaN if a NaN was seen)
     float lse_s;    // sum of 2^((z - m) * c2)
     uint32_t count; // entries that follow: rank keys, best first
-    uint32_t flags; // bit 0: the shard held more than `count` candidates; bit 1: the record is not exact
+    uint32_t flags; // bit 0: the shard held more than `count` candidates; bit 1: the pass over the shard failed (no entries)
     float bound;
     uint32_t pad[3];
 };
@@ -890,6 +890,15 @@ __device__ __forceinline__ void write_packed(const ScanArgs& A, ScanShared& sh, 
         h.pad[0] = h.pad[1] = h.pad[2] = 0;
         memcpy(rec, &h, sizeof h);
     }
+}
+
+// The record of a virtual row that could not be streamed: the merge reports the failure instead of
+// sampling whatever the record's place held before.  One thread.
+__device__ __forceinline__ void write_failed(const ScanArgs& A, int b, int g) {
+    PackedHdr h;
+    h.m = -INFINITY; h.lse_s = 0.0f; h.count = 0; h.flags = 2u; h.bound = -INFINITY;
+    h.pad[0] = h.pad[1] = h.pad[2] = 0;
+    memcpy(A.packed + (int64_t)g * A.packed_seg_stride + (int64_t)b * A.packed_row_stride, &h, sizeof h);
 }
 
 template <typename T>

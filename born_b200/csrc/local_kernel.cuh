@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) local_kernel(const __grid_con
             if (nl) flush();
             if (n > kLocalCap) {  // (many equal values): the exact search, at the end
                 if (lane == 0) {
+                    write_failed(A, q.b, q.g);  // (should a wait of another warp run out)
                     A.deferred[r] = (8u << 24) | (blockIdx.x + 1u);
                     sh.defer = 1;
                 }
@@ -214,6 +215,10 @@ __global__ void __launch_bounds__(kScanThreads, 2) local_kernel(const __grid_con
     if (failed) {
         // a wait ran out: the copies still in flight (all but the one the test hook withheld) get the same bounded wait
         if (lane == 0) atomicExch(A.dev_error, BORN_ERR_DEVICE_TIMEOUT);
+        for (int x = r + lane * W; x < R; x += 32 * W) {
+            const RowGeom q = row_geom<T>(A, x);
+            write_failed(A, q.b, q.g);
+        }
         while (r < R && (r != ri || j != ji)) {
             if ((long long)r * nb + j != A.debug_skip_blk) ring_wait(bar0 + sc * (kScanWarps * 8u), phase, A.timeout_ns);
             if (++sc == (uint32_t)S) { sc = 0; phase ^= 1u; }

@@ -41,14 +41,14 @@ __global__ void __launch_bounds__(kThreads) merge_kernel(const __grid_constant__
     // records with a read and an atomic each was a chain of G round trips to L2.)
     const int lane = tid & 31, warp = tid >> 5;
     float m = -INFINITY, ls = 0.0f;
-    int cnt = 0, inexact = 0;
+    int cnt = 0, failed = 0;
     if (tid == 0) sh.nl = 0;
     if (lane < A.G) {
         const uint32_t* h = reinterpret_cast<const uint32_t*>(rec_of(lane));
         m = __uint_as_float(__ldcg(h));
         ls = __uint_as_float(__ldcg(h + 1));
-        cnt = (int)__ldcg(h + 2);
-        inexact = (int)(__ldcg(h + 3) & 2u);
+        cnt = (int)min(__ldcg(h + 2), (uint32_t)((A.row_stride - kRecordHdrBytes) / 8));  // (never beyond the record)
+        failed = (int)(__ldcg(h + 3) & 2u);
     }
     cta_sync();
     const float mg = m;
@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(kThreads) merge_kernel(const __grid_constant__
     ls = ls > 0.0f ? ls * ex2_approx(__fmul_rn(mg - m, c2)) : 0.0f;
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, d);
-    inexact = __any_sync(0xffffffffu, inexact);
+    failed = __any_sync(0xffffffffu, failed);
     for (int g = warp; g < A.G; g += kScanWarps) {
         const int c = __shfl_sync(0xffffffffu, cnt, g);
         const unsigned long long* ent = reinterpret_cast<const unsigned long long*>(rec_of(g) + kRecordHdrBytes);
@@ -85,10 +85,11 @@ __global__ void __launch_bounds__(kThreads) merge_kernel(const __grid_constant__
     o.kept_ids = A.out_kept_ids; o.kept_count = A.out_kept_count; o.kept_stride = A.kept_stride;
     o.row = b;
     int status = BORN_ROW_OK;
-    if (m != m) status = BORN_ROW_NAN;
+    if (failed) status = 100 + BORN_ERR_DEVICE_TIMEOUT;
+    else if (m != m) status = BORN_ROW_NAN;
     else if (m == INFINITY) status = BORN_ROW_POS_INF;
     else if (m == -INFINITY) status = BORN_ROW_ALL_MASKED;
-    else if (inexact || n > kSelCap) status = BORN_ROW_OVERFLOW;
+    else if (n > kSelCap) status = BORN_ROW_OVERFLOW;
     if (A.out_lse && tid == 0) A.out_lse[b] = (status == BORN_ROW_OK || status == BORN_ROW_OVERFLOW) ? m * inv_T + __log2f(ls) * 0.69314718f : NAN;
     if (status != BORN_ROW_OK) {
         row_fail(o, status);

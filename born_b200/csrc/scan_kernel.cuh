@@ -611,11 +611,13 @@ __global__ void __launch_bounds__(kScanThreads, 2) scan_kernel(const __grid_cons
             if (tt != A.debug_skip_blk) ring_wait(bar0 + sc * (kScanWarps * 8u), phase, A.timeout_ns);
             if (++sc == (uint32_t)S) { sc = 0; phase ^= 1u; }
         }
-        const int r0 = (int)(t0 / nb), r1 = (int)((t1 - 1) / nb);
+        const int r0 = (int)(t0 / nb), r1 = (int)((t1 - 1) / nb), rf = (int)(t / nb);
         for (int r = r0 + tid; r <= r1; r += kThreads) {
             if (A.mode == kScanFull) {
                 A.out_status[r / A.G] = 100 + BORN_ERR_DEVICE_TIMEOUT;
                 A.out_token[r / A.G] = -1;
+            } else if (r >= rf) {  // (an earlier row's record is written, or another CTA's to write)
+                write_failed(A, r / A.G, r % A.G);
             }
         }
         return;

@@ -56,7 +56,7 @@ extern "C" {
 #define BORN_ROW_ALL_MASKED 1 /* no allowed token with a logit above -inf: token = -1 */
 #define BORN_ROW_NAN 2        /* NaN logit among the allowed tokens: token = -1 */
 #define BORN_ROW_POS_INF 3    /* +inf logit among the allowed tokens: token = -1 */
-#define BORN_ROW_OVERFLOW 4   /* only from the vocab-sharded path: a shard record could not be made exact */
+#define BORN_ROW_OVERFLOW 4   /* only from born_shard_merge: the gathered records hold more than BORN_MAX_CANDIDATES tokens */
 #define BORN_ROW_BAD_TOKEN 5  /* speculative verify: draft token outside [0, vocab) */
 #define BORN_ROW_BAD_PARAMS 7 /* a row of a device-resident row_params array is out of range: token = -1 */
 #define BORN_ROW_FINISHED 6   /* born_sample_next: the row sampled a stop token in an earlier step; token = -1 */
@@ -252,10 +252,11 @@ int32_t born_last_timing(void* handle, float* out3);
 const char* born_last_error(void* handle);
 const char* born_version(void);
 
-/* Test hook: one small sampling launch in which one bulk copy is withheld and the wait limit
- * is a millisecond, so that the bounded wait gives up.  Returns BORN_ERR_DEVICE_TIMEOUT when
- * the kernel reported the expiry and came back (the expected outcome), BORN_OK when it did
- * not expire.  The handle stays usable.  Synchronises the stream. */
+/* Test hook: small launches of every work decomposition (a CTA per row, clusters, slices, ranges, a
+ * warp per row) in each of which one bulk copy is withheld and the wait limit is a millisecond, so
+ * that the bounded wait gives up.  Returns BORN_ERR_DEVICE_TIMEOUT when every launch reported the
+ * expiry, came back and left the right rows failed (the expected outcome), BORN_OK when one did not
+ * expire.  The handle stays usable.  Synchronises the stream. */
 int32_t born_debug_expire_wait(void* handle, void* stream);
 
 /* ---- the autoregressive loop around the sampler ---------------------------------------

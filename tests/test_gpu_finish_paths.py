@@ -139,3 +139,36 @@ def test_warp_per_row_segments(sampler, oracle, V, G, k, dtype):
         truth = x.max() + np.log(np.exp(x - x.max()).sum())
         # 1e-5 relative on sum(exp) is 1e-5 absolute on its logarithm
         assert abs(got["lse"][b] - truth) <= 1e-5 + 1e-6 * abs(truth), (b, got["lse"][b], truth)
+
+
+# a wait that runs out in every work decomposition leaves the right rows failed (the hook checks the statuses)
+# and nothing behind: records, tickets, deferred rows
+def test_expired_waits_of_every_decomposition(sampler, oracle, lib):
+    from born_b200 import _lib as L
+    rc = lib.born_debug_expire_wait(sampler._h, None)
+    assert rc == L.ERR_DEVICE_TIMEOUT, (rc, lib.born_last_error(sampler._h))
+    for B, V, G in ((2, 49152, 1), (301, 50176, 1), (100, 2048 * 8, 8)):
+        z = _logits(B, B, V, "f32")
+        got, ref = run_both(sampler, oracle, z, dict(temperature=1.0, top_k=16), W.uniform_f32(B, 2, B), segments=G)
+        assert_parity(got, ref)
+    sampler.check_error()
+
+
+# a gathered record of a pass that failed fails its row; a count beyond the record reads no further than it
+def test_merge_of_failed_and_overlong_records(sampler):
+    import torch
+    from born_b200 import _lib as L
+    B, V, K, G = 5, 4096, 16, 2
+    z = torch.from_numpy(_logits(77, B, V * G, "f32")).cuda()
+    u = torch.from_numpy(W.uniform_f32(77, 2, B)).cuda()
+    gathered = torch.stack([sampler.shard_local(z[:, g * V:(g + 1) * V], g, G, K) for g in range(G)])
+    want = {k: v.clone() for k, v in sampler.shard_merge(gathered, u, V, 0, G, K).items()}
+    words = gathered.view(torch.int32)
+    words[1, 2, 2] = 0x7FFFFFFF
+    words[0, 3, 2] = -1
+    words[1, 4, 3] |= 2
+    got = sampler.shard_merge(gathered, u, V, 0, G, K)
+    assert (want["status"] == L.ROW_OK).all()
+    for k in ("token", "status", "prob", "lse"):
+        assert torch.equal(got[k][:4], want[k][:4]), k
+    assert got["status"][4] == 100 + L.ERR_DEVICE_TIMEOUT and got["token"][4] == -1 and torch.isnan(got["lse"][4])
