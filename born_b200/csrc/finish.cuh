@@ -410,7 +410,7 @@ __device__ __forceinline__ float token_logit(const ScanArgs& A, const born_row_p
         const int32_t* gh = A.history + (int64_t)b * A.history_stride;
         const int id = g * A.V + tok;
         int cnt = 0;
-        for (int p = 0; p < len; ++p) cnt += (__ldcg(gh + p) == id) ? 1 : 0;  // (hist_ids: not read-only)
+        for (int p = 0; p < len; ++p) cnt += (gh[p] == id) ? 1 : 0;  // (plain reads, cached in L1: hist_ids has why not read-only ones)
         if (cnt > 0) z = penalise(rp, z, cnt);
     }
     if (A.mask) {
