@@ -522,11 +522,13 @@ constexpr float kBinScale = 32.0f;
 __device__ __forceinline__ int nucleus_bin(float z, float m, float inv_T) {
     return (int)fminf(__fmul_rn(__fmul_rn(__fsub_rn(m, z), inv_T), kBinScale), (float)(kBins - 1));
 }
+template <bool kTakeOut = false>
 __device__ __forceinline__ void bin_mass(uint32_t* limb, int bin, uint64_t q) {
     if (q == 0) return;
-    smem_red_add(&limb[bin], (uint32_t)q & 0x3FFFu);
-    smem_red_add(&limb[kBins + bin], (uint32_t)(q >> 14) & 0x3FFFu);
-    if (q >> 28) smem_red_add(&limb[2 * kBins + bin], (uint32_t)(q >> 28));
+    auto add = [&](uint32_t* p, uint32_t part) { smem_red_add(p, kTakeOut ? 0u - part : part); };
+    add(&limb[bin], (uint32_t)q & 0x3FFFu);
+    add(&limb[kBins + bin], (uint32_t)(q >> 14) & 0x3FFFu);
+    if (q >> 28) add(&limb[2 * kBins + bin], (uint32_t)(q >> 28));
 }
 __device__ __forceinline__ uint64_t bin_total(const uint32_t* limb, int bin) {
     return (uint64_t)limb[bin] + ((uint64_t)limb[kBins + bin] << 14) + ((uint64_t)limb[2 * kBins + bin] << 28);
@@ -995,7 +997,8 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
             draw_whole_row<T>(A, sh, o, rp, b, g, row, m, pl.inv_T, S_tot, src.u);
             return;
         }
-        if (kHist && penalties_on(rp)) {  // (the bins below would have to look every token up in the history)
+        const bool pen = kHist && penalties_on(rp);
+        if (pen && sizeof(T) == 2) {  // (group keys without the history tokens; such rows come here as an fp32 copy)
             if (tid == 0) defer_row(A, sh, row, 7u);
             return;
         }
@@ -1034,9 +1037,20 @@ __device__ __forceinline__ void finish_row(const ScanArgs& A, ScanShared& sh, ui
                         mass2_of(make_float2(z[e], z[e + 1]), m, pl.inv_T, q[0], q[1]);
 #pragma unroll
                         for (int h = 0; h < 2; ++h)
-                            if (z[e + h] >= cut) bin_mass(limb, nucleus_bin(z[e + h], m, pl.inv_T), q[h]);
+                            if (z[e + h] >= cut && (!pen || z[e + h] <= m)) bin_mass(limb, nucleus_bin(z[e + h], m, pl.inv_T), q[h]);
                     }
                 });
+                if (pen) {
+                    const uint8_t* base = reinterpret_cast<const uint8_t*>(A.logits) + ((int64_t)b * A.row_stride + (int64_t)g * A.V) * (int64_t)sizeof(T);
+                    for_history(A, smem, src, [&](int tok, float zp) {
+                        const float z = raw_logit<T>(base, tok);
+                        uint64_t q, qp;
+                        mass2_of(make_float2(z, zp), m, pl.inv_T, q, qp);
+                        if (z >= cut && z <= m && zp > -INFINITY && (uint32_t)src.gkeys[tok / kGrpTok] >= zkey(cut) >> 16)
+                            bin_mass<true>(limb, nucleus_bin(z, m, pl.inv_T), q);
+                        if (zp >= cut) bin_mass(limb, nucleus_bin(zp, m, pl.inv_T), qp);
+                    });
+                }
             }
             cta_sync();
             if (tid == 0) sh.ng[0] = sh.ng[1] = 0;  // (for the candidates' own round)

@@ -101,6 +101,36 @@ def test_history_tokens_among_the_candidates(sampler, oracle, B, dtype):
         assert_parity(got, ref)
 
 
+# top-p alone over penalised values: from the group keys (peaked rows), from the groups' tokens or by the exact search
+# (flat ones); history tokens above the penalised maximum,
+# raised by a penalty below zero, masked, and beside the nucleus
+@pytest.mark.parametrize("B,V,masked", [(1, 50176, False), (24, 50176, False), (24, 50176, True), (200, 16384, False), (301, 50176, False),
+                                        (400, 8192, True)])
+def test_nucleus_of_penalised_rows(sampler, oracle, B, V, masked):
+    H = 200
+    rank = np.argsort(W.uniform_f32(B, 4, B * V).reshape(B, V), axis=1).argsort(axis=1)
+    z = _logits(B + V, B, V, "f32", 1.0) - np.float32(1.6) * np.log(rank + 1.0).astype(np.float32)
+    flat = np.arange(B) % 8 == 7
+    z[flat] = _logits(B + V, B, V, "f32", 2.2)[flat]
+    order = np.argsort(-z, axis=1)
+    hist = W.randint(B, 5, B * H, V).astype(np.int32).reshape(B, H)
+    hist[:, :40] = order[:, :80:2]
+    hist[:, 40:60] = order[:, :40:2]
+    mask = None
+    if masked:
+        bits = W.uniform_f32(B, 6, B * V).reshape(B, V) < 0.7
+        bits[:, 0] = True
+        mask = np.packbits(bits, axis=1, bitorder="little").view(np.uint32)
+    u = W.uniform_f32(B, 2, B)
+    for params in (dict(temperature=0.8, top_p=0.9, repetition_penalty=1.2), dict(temperature=1.1, top_p=0.6, frequency_penalty=-0.7),
+                   dict(temperature=0.6, top_p=0.97, repetition_penalty=1.1, frequency_penalty=0.5, presence_penalty=0.3)):
+        sampler.fallback_rows
+        got, ref = run_both(sampler, oracle, z, params, u, mask=mask, hist=hist, want_kept=1024)
+        assert_parity(got, ref)
+        # only the flat rows, whose nucleus or its bound may not fit the selection, take the exact search
+        assert sampler.fallback_rows <= flat.sum()
+
+
 # more rows than CTAs fit at once: a CTA per row in waves, and ranges for long rows with a nearly empty second wave
 @pytest.mark.parametrize("B,V,dtype", [(297, 1000, "f32"), (301, 50176, "f32"), (303, 50001, "bf16"), (375, 50176, "bf16"), (600, 1031, "bf16")])
 def test_more_rows_than_fit_at_once(sampler, oracle, B, V, dtype):
