@@ -588,7 +588,7 @@ __device__ __forceinline__ uint32_t kth_of_maxima(const uint32_t (&v)[8], int k)
 // take four and 2.3 us).
 // Larger k, or too few threads with a live key: bins -- equal steps of the value below the maximum m --
 // down to the smallest of the threads' maxima (at least as many keys as threads reach that).  All
-// threads get the same answer; kDeadKey16 + 1 when fewer than k are alive.
+// threads get the same answer; kDeadKey16 + 1 when fewer than k are alive.  `bins`: 2 x kBins words.
 template <typename F>
 __device__ __forceinline__ uint32_t kth_key(F key_of, int n, int k, float m, uint32_t* bins, ScanShared& sh) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -619,7 +619,9 @@ __device__ __forceinline__ uint32_t kth_key(F key_of, int n, int k, float m, uin
     for (int g = tid + kReg * kThreads; g < n; g += kThreads) see(key_of(g));
     const uint32_t lo_w = __reduce_min_sync(0xffffffffu, mx), mn_w = __reduce_min_sync(0xffffffffu, mn);
     if (lane == 0) sh.redu[warp] = (lo_w << 16) | mn_w;
+    uint32_t* least = bins + kBins;
     reinterpret_cast<uint4*>(bins)[tid] = make_uint4(0u, 0u, 0u, 0u);
+    reinterpret_cast<uint4*>(least)[tid] = make_uint4(~0u, ~0u, ~0u, ~0u);
     cta_sync();
     uint32_t lo = 0xFFFFu;
     mn = 0xFFFFu;
@@ -633,13 +635,15 @@ __device__ __forceinline__ uint32_t kth_key(F key_of, int n, int k, float m, uin
     const float span = m - zkey_to_float(lo << 16);
     const float scale = span > 0.0f ? (float)(kBins - 1) / span : 0.0f;
     auto bin_of = [&](uint32_t key) { return (int)fminf(__fmul_rn(m - zkey_to_float(key << 16), scale), (float)(kBins - 1)); };
+    auto count = [&](uint32_t key) {
+        if (key < lo) return;
+        const int bin = bin_of(key);
+        smem_red_add(&bins[bin], 1u);
+        smem_red_min(&least[bin], key);
+    };
 #pragma unroll
-    for (int i = 0; i < kReg; ++i)
-        if (kk[i] >= lo) smem_red_add(&bins[bin_of(kk[i])], 1u);
-    for (int g = tid + kReg * kThreads; g < n; g += kThreads) {
-        const uint32_t key = key_of(g);
-        if (key >= lo) smem_red_add(&bins[bin_of(key)], 1u);
-    }
+    for (int i = 0; i < kReg; ++i) count(kk[i]);
+    for (int g = tid + kReg * kThreads; g < n; g += kThreads) count(key_of(g));
     cta_sync();
     const uint4 c = reinterpret_cast<const uint4*>(bins)[tid];
     uint32_t incl = c.x + c.y + c.z + c.w;
@@ -665,21 +669,10 @@ __device__ __forceinline__ uint32_t kth_key(F key_of, int n, int k, float m, uin
     cta_sync();
     const int b = sh.found;
     if (b < 0) return kDeadKey16 + 1u;
-    if (b == kBins - 1 || scale == 0.0f) return lo;
-    // The smallest key that was counted into the bins up to b: k keys reach it by that count.  (An edge
-    // worked back from the bin's number would carry the rounding of m - z, half a unit in the last place of
-    // m, which is many steps of a key that is small beside m.)
-    uint32_t low = 0xFFFFu;
-    auto counted = [&](uint32_t key) { low = key >= lo && bin_of(key) <= b ? min(low, key) : low; };
-#pragma unroll
-    for (int i = 0; i < kReg; ++i) counted(kk[i]);
-    for (int g = tid + kReg * kThreads; g < n; g += kThreads) counted(key_of(g));
-    low = __reduce_min_sync(0xffffffffu, low);
-    if (lane == 0) sh.redu[warp] = low;
-    cta_sync();
-#pragma unroll
-    for (int w = 0; w < kScanWarps; ++w) low = min(low, sh.redu[w]);
-    return low;
+    // The smallest key counted into the crossing bin: the bins follow the order of the keys, so k keys reach
+    // it by that count.  (An edge worked back from the bin's number would carry the rounding of m - z, half a
+    // unit in the last place of m, which is many steps of a key that is small beside m.)
+    return least[b];
 }
 
 // Raw logit of token `tok` of the row at `base` (no mask, no penalties).

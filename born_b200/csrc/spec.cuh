@@ -132,6 +132,9 @@ __device__ __forceinline__ uint32_t smem_atom_add(void* p, uint32_t v) {
 __device__ __forceinline__ void smem_red_add(void* p, uint32_t v) {
     asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
 }
+__device__ __forceinline__ void smem_red_min(void* p, uint32_t v) {
+    asm volatile("red.shared.min.u32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
+}
 __device__ __forceinline__ void smem_red_or(void* p, uint32_t v) {
     asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
 }
