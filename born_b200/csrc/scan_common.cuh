@@ -31,6 +31,8 @@ constexpr int kScanStagesMax = 8;           // slots per warp ring, at most
 constexpr int kMassBlock = 512;             // tokens per mass block of the whole-vocabulary routes: half a warp's block
 constexpr int kSelCap = 1024;               // candidates the in-shared-memory selection handles
 constexpr int kHistBuckets = 128;           // the history list of a segment is grouped by block (or run of blocks)
+constexpr int kHistTables = 32768;          // ... built with tables of this size where the ring has the room
+constexpr int kHistPos = 2048;              // ... and this many list positions by a hash of the token
 constexpr int kClusterMax = 8;              // slices of a row that exchange through distributed shared memory
 constexpr int kGrpRound = 4096;             // group keys a CTA looks at before it reads the groups it found again
 constexpr int kBins = 1024;                 // bins of the finish's histograms
@@ -63,9 +65,11 @@ struct ScanSmem {
     int stages;     // ring slots per warp
     int slot;       // bytes per slot: logits, then the mask words
     int work;       // kWorkBytes for the finish.  One segment per CTA: over the ring, idle by then
-    int hash;       // the history build's table: 2^hash_lg keys and counts.  One segment per CTA: the
-                    // last ring stage, which is filled only after the build; else the work area
-    int hash_lg;
+    int hash;       // the history build's tables (hist_build).  One segment per CTA: the last `held` ring
+                    // stages, which are filled only after the build; else the work area
+    int hash_lg;    // ... 2^hash_lg keys and counts fit
+    int hash_bytes; // ... room there is
+    int held;
     int gkeys;      // group keys of a row the CTA streams alone ...
     int gkeys_cap;  // ... groups there is room for
     int list;       // history list, then the kHistBuckets + 1 bucket offsets
@@ -193,11 +197,16 @@ inline ScanSmem scan_smem_layout(int elem_bytes, bool aligned, bool has_mask, in
     int off = L.stages * stage;
     if (one_seg) {
         L.work = 0;
-        L.hash = (L.stages - 1) * stage;
+        L.held = hist_cap ? (kHistTables + stage - 1) / stage : 0;
+        if (L.held > L.stages - 1) L.held = L.stages - 1;
+        L.hash = (L.stages - L.held) * stage;
+        L.hash_bytes = L.held * stage;
     } else {
         L.work = off;
         off += kWorkBytes;
         L.hash = L.work;
+        L.hash_bytes = kWorkBytes;
+        L.held = 0;
     }
     if (off < kExactBytes) off = kExactBytes;
     L.gkeys = off;

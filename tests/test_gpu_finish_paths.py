@@ -101,6 +101,27 @@ def test_history_tokens_among_the_candidates(sampler, oracle, B, dtype):
         assert_parity(got, ref)
 
 
+# the history list by bits (up to the longest segment whose bits fit the ring) and by the hash table (beyond it,
+# and in ranges of long rows): few tokens many times each, tokens that share a hash, ids outside the row
+@pytest.mark.parametrize("B,V,dtype", [(2, 1000, "f32"), (40, 32001, "f32"), (150, 229376, "bf16"), (150, 229377, "bf16"), (150, 262144, "f32"),
+                                       (300, 180000, "bf16")])
+def test_history_list_by_bits_and_by_hash(sampler, oracle, B, V, dtype):
+    H = 700
+    z = _logits(V, B, V, dtype)
+    val = z if dtype == "f32" else (z.astype(np.uint32) << 16).view(np.float32)
+    hist = W.randint(V, 4, B * H, V).astype(np.int32).reshape(B, H)
+    top = np.argpartition(-val, 50, axis=1)[:, :50]
+    hist[:, :50] = top
+    hist[:, 50:100] = top[:, ::-1]                   # repeats
+    hist[:, 100:400] = hist[:, 300:600]              # ... of tokens all over the row, many with a common hash
+    hist[:, 600:680] = top[:, :1]                    # one token many times
+    hist[:, 680:690], hist[:, 690:] = -1, V
+    for params in (dict(temperature=0.9, top_k=40, repetition_penalty=1.2, frequency_penalty=0.02),
+                   dict(temperature=0.9, min_p=0.05, top_p=0.9, frequency_penalty=0.05, presence_penalty=0.3)):
+        got, ref = run_both(sampler, oracle, z, params, W.uniform_f32(V, 2, B), hist=hist)
+        assert_parity(got, ref)
+
+
 # top-p alone over penalised values: from the group keys (peaked rows), from the groups' tokens or by the exact search
 # (flat ones); history tokens above the penalised maximum,
 # raised by a penalty below zero, masked, and beside the nucleus
