@@ -480,8 +480,9 @@ int64_t born_fallback_rows(void* handle) {
     int n[24];
     if (cudaMemcpy(n, h->dev_error + 1, sizeof n, cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
     cudaMemset(h->dev_error + 1, 0, sizeof n);
-    // by reason: 1 greedy tie lost, 2 kept-id list of a whole row, 3 more than 1024 candidates, 4 top-k above 256,
-    // 5 / 6 top-k / min-p set not provably complete, 7 nucleus below the candidates, 8 shard record not exact
+    // by reason: 2 kept-id list of a whole row; more than 1024 candidates for 1 greedy (ties), 5 top-k, 6 min-p;
+    // 7 top-p alone: more than 1024 candidates, or a nucleus that reaches below them; 8 a virtual row with
+    // more candidates than its selection holds (3 and 4 are not in use)
     snprintf(h->err, sizeof h->err, "exact-search rows by reason 1..8: %d %d %d %d %d %d %d %d", n[8], n[9], n[10], n[11], n[12],
              n[13], n[14], n[15]);
     return n[0];

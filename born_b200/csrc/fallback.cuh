@@ -12,9 +12,7 @@
 // from L2.  A pass takes a warp through the row's blocks: the group keys of a block (where the row
 // still has them) say which of its 32 groups are read at all.
 //
-// What bounds it is the one CTA's issue rate: 0.6 us per pass and 10 000 tokens.  (Before: five passes
-// of 4096 shared-memory bins through a staging buffer and one more with a block scan per 4096
-// tokens; 128256-token rows took 1.0 to 1.2 ms.)
+// What bounds it is the one CTA's issue rate: 0.6 us per pass and 10 000 tokens.
 #pragma once
 #include "scan_common.cuh"
 #include "finish.cuh"

@@ -51,8 +51,8 @@ struct SelectIn {
 // Threads that share the loops over one of n candidates: log2.  The loops are chains of
 // shared-memory reads, so the CTA's 256 threads are dealt over (candidate, part of the loop).
 __device__ __forceinline__ int split_lg(int n) { return n <= 32 ? 3 : n <= 64 ? 2 : n <= 128 ? 1 : 0; }
-// Candidates up to which every one is compared with every other (select_small).  The comparisons are quadratic:
-// 200 candidates took 13.4 us of a merge launch that sorts 400 in 9.9.
+// Candidates up to which every one is compared with every other (select_small).  The comparisons are quadratic: a
+// merge launch over 200 candidates takes 13.4 us with them, one that sorts 400 takes 9.9.
 constexpr int kSmallMax = 128;
 
 // Selection and draw over n <= kSmallMax candidates in shared memory (sel: rank keys; selq: scratch for
@@ -201,7 +201,7 @@ __device__ __forceinline__ int find_bin(F total_of, unsigned long long target, u
 // Selection and draw over kSmallMax < n <= kSelCap candidates, the same rules, four candidates per thread.
 // A counting sort puts them in rank order: bins of equal width in value from the best candidate down,
 // places inside a bin by comparison.  Then the masses are scanned in rank order, and the draw finds its
-// token through bins of the token index.  (Three radix descents, over keys, masses and indices, took
+// token through bins of the token index.  (Three radix descents, over keys, masses and indices, take
 // 18 us for 300 candidates.)  `bins`: kBins 64-bit words.
 static __device__ __noinline__ bool select_large(const SelectIn in, uint64_t* sel, unsigned long long* selq, uint32_t* bins,
                                                  ScanShared& sh, const RowOut o) {

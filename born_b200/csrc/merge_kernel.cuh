@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kThreads) merge_kernel(const __grid_constant__
     auto rec_of = [&](int g) { return A.gathered + (int64_t)g * A.seg_stride + (int64_t)b * A.row_stride; };
     // Every warp folds the headers for itself, a lane per record (word by word: a record of an odd number
     // of entries is only 8-byte aligned); then the warps share out the records' entries.  (A loop over the
-    // records with a read and an atomic each was a chain of G round trips to L2.)
+    // records with a read and an atomic each is a chain of G round trips to L2.)
     const int lane = tid & 31, warp = tid >> 5;
     float m = -INFINITY, ls = 0.0f;
     int cnt = 0, failed = 0;

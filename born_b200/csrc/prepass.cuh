@@ -1,9 +1,9 @@
 // Clean-copy prepass.  The whole-vocabulary routes of scan_kernel form their mass blocks on
-// 512-token blocks aligned to the row start, inside the warps' fixed tile slices.  Rows that
-// do not start on a 16-byte boundary, and bf16 rows with history penalties (a bf16 tile cannot
-// hold a penalised fp32 value), are therefore first written to a 16-byte-aligned fp32 copy with
-// the grammar mask and the penalties already applied -- the same operations in the same order
-// as everywhere else: upcast, repetition (z > 0 ? z / r : z * r), z - (frequency * count +
+// 512-token blocks aligned to the row start, half a warp each (instantiated for 16-byte-aligned rows
+// only), and a bf16 slot cannot hold a penalised fp32 value.  Rows that do not start on a 16-byte
+// boundary, and bf16 rows with history penalties, are therefore first written to a 16-byte-aligned
+// fp32 copy with the grammar mask and the penalties already applied -- the same operations in the
+// same order as everywhere else: upcast, repetition (z > 0 ? z / r : z * r), z - (frequency * count +
 // presence), then -inf where the mask bit is clear.
 #pragma once
 #include "scan_common.cuh"

@@ -10,10 +10,8 @@
 // online log-sum-exp, and stores one 16-bit key per lane.  The k-th largest group maximum is
 // reached by at least k tokens, so the groups that reach it hold the k best tokens; a group below
 // running maximum + delta holds no min-p survivor; and so on for every route -- decided once, in the
-// finish, when everything is known.  (The design before this one compared every value with
-// thresholds that tightened while the row streamed and pushed hits into 256-entry buffers: nine
-// iterations in ten took the hit path for top-k, and a full buffer sent the row to an exact search
-// of a millisecond.)
+// finish, when everything is known.  (Thresholds that tighten while the row streams, with hits pushed
+// into buffers, send nine iterations in ten down the hit path for top-k.)
 //
 // 8 warps per CTA, two CTAs per SM, no producer warp: warp_ring.cuh.  What bounds it on long
 // rows is HBM; on one-block-per-warp rows the chain launch -> history list -> copy -> reduction ->

@@ -42,9 +42,8 @@ __device__ __forceinline__ bool ck_alive(uint64_t ck) { return (ck >> 24) != 0; 
 // Same operation sequence as the CPU oracle: Cody-Waite reduction, degree-6 polynomial,
 // exponent-field scaling.  x <= 0; returns 0 below -80 and for NaN.
 // kSelect: no branch -- an argument below -80, or NaN, runs the arithmetic on -80 and selects 0 at the
-// end; otherwise those arguments return early.  Same bits either way; which one is faster depends
-// on the caller (measured: the select form takes 3 % off the whole-vocabulary rows of the streaming
-// kernel and adds 2 % to the verify kernels, which therefore ask for the branch).
+// end; otherwise those arguments return early.  Same bits either way.  The streams' inner loops take the
+// packed form below; this one serves single tokens and block totals.
 template <bool kSelect = true>
 __device__ __forceinline__ float exp_det(float x) {
     const bool in_range = x >= -80.0f;

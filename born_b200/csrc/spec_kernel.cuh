@@ -96,9 +96,9 @@ __device__ __forceinline__ void draw_weight2(const DrawCtx& D, float2 zp, float2
 // The blocks of all rows form one sequence, dealt to all warps of the grid in contiguous, equal
 // ranges; a warp streams its blocks through its own ring (warp_ring.cuh) and never meets another
 // warp.  Bound by the fp32 pipe and issue slots of the deterministic exp (13 instructions per token
-// in packed form, 27 before), then by HBM: one pass, every logit read once.  32 sequences of five
-// draft tokens over 128256-token rows (180.6 MB): 90.6 us before, 53.0 us now, both launches; tiles
-// of 8192 tokens behind a block-wide barrier each had left the pipes idle while the warps met.
+// in packed form, 27 in scalar), then by HBM: one pass, every logit read once.  32 sequences of five
+// draft tokens over 128256-token rows (180.6 MB): 55.6 us, both launches, against 94 with tiles of 8192
+// tokens behind a block-wide barrier each, which leave the pipes idle while the warps meet.
 struct MassShared {
     unsigned long long bars[kSpecStages * (kSpecThreads / 32)];
 };
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kSpecThreads, 2) spec_mass_kernel(const __grid
 // a block's sum stays inside its warp -- the operands of the accept tests are fetched before the
 // block results are waited for, and the launch itself overlaps the first one's end (programmatic
 // dependent launch: everything in front of grid_dependency_wait reads only the caller's inputs).
-// Four sequences of four draft tokens, 18917-token rows: 26.5 us for both launches before, 12.7 us now.
+// Four sequences of four draft tokens, 18917-token rows: 12.7 us for both launches, 26.5 with block-wide steps.
 struct DrawShared {
     unsigned long long rowS[kSpecMaxRows];   // row totals of the fixed-point masses
     unsigned long long csum[kSpecMaxBlocks];

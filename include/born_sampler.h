@@ -185,8 +185,8 @@ int32_t born_sampler_destroy(void* handle);
  * every logit is read once, whatever the parameters (per-row parameter arrays included).
  * Rows whose kept set is small (top-k, min-p, a nucleus of up to 1024 tokens) are finished
  * from the candidates collected while streaming; rows that nothing narrows are drawn from
- * exact per-512-token mass blocks; any other row (top-k above 256, a nucleus or a min-p
- * survivor set beyond 1024 tokens) takes an exact multi-pass search inside the same launch --
+ * exact per-512-token mass blocks; any other row (a nucleus, a min-p survivor set or ties at the
+ * top-k threshold beyond 1024 tokens) takes an exact multi-pass search inside the same launch --
  * slower, never approximate.  Two more launches come first when whole-vocabulary rows are not
  * 16-byte aligned or are bf16 with history penalties (see "Ownership" above). */
 int32_t born_sample(void* handle, const born_sample_args* args, void* stream);
@@ -239,7 +239,7 @@ int32_t born_sample_static(const born_sample_args* args, void* stream);
 /* No counterpart in the reference.  Rows that took the exact multi-pass search (see
  * born_sample) since the last call of this function; synchronises the device.  A serving
  * loop can watch it: a workload whose rows keep landing there is paying for a flat
- * distribution (or a top-k above 256), not for a fault. */
+ * distribution, not for a fault. */
 int64_t born_fallback_rows(void* handle);
 
 /* Bytes of device workspace a handle holds (for capacity planning). */

@@ -122,6 +122,27 @@ def test_history_list_by_bits_and_by_hash(sampler, oracle, B, V, dtype):
         assert_parity(got, ref)
 
 
+# a cluster whose rows are too long for their group keys to stay in shared memory
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_cluster_with_keys_in_global_memory(oracle, dtype):
+    from born_b200 import Sampler
+    B, V, H = 2, 450000, 100
+    z, u = _logits(45, B, V, dtype, 4.0), W.uniform_f32(45, 2, B)
+    val = z if dtype == "f32" else (z.astype(np.uint32) << 16).view(np.float32)
+    hist = W.randint(45, 4, B * H, V).astype(np.int32).reshape(B, H)
+    hist[:, :40] = np.argsort(-val, axis=1)[:, :80:2]
+    s = Sampler(device=0, max_batch=B, max_vocab=V)
+    try:
+        for params in (dict(temperature=1.0, top_k=50), dict(temperature=1.0, top_k=200, top_p=0.9), dict(temperature=0.8, min_p=0.05),
+                       dict(temperature=0.5, top_p=0.8), dict(temperature=0.0)):
+            for h in (None, hist):
+                p = dict(params, **({} if h is None else dict(repetition_penalty=1.2)))
+                got, ref = run_both(s, oracle, z, p, u, hist=h)
+                assert_parity(got, ref)
+    finally:
+        s.close()
+
+
 # top-p alone over penalised values: from the group keys (peaked rows), from the groups' tokens or by the exact search
 # (flat ones); history tokens above the penalised maximum,
 # raised by a penalty below zero, masked, and beside the nucleus
@@ -169,7 +190,9 @@ def test_more_rows_than_fit_at_once(sampler, oracle, B, V, dtype):
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("V,G,k", [(520, 8, 8), (1024, 8, 16), (1032, 8, 16), (8200, 8, 64), (9216, 8, 128), (9016, 4, 1)])
 def test_warp_per_row_segments(sampler, oracle, V, G, k, dtype):
-    B = 752 // G
+    import torch
+    # (a CTA per row would take more than two waves and a half of two per SM)
+    B = -(-(5 * torch.cuda.get_device_properties(0).multi_processor_count + 8) // G)
     z = _logits(V + k, B, V * G, dtype)
     ninf, pinf, nan, one = ((np.float32(x) for x in (-np.inf, np.inf, np.nan, 1.0)) if dtype == "f32" else
                             (np.uint16(x) for x in (0xFF80, 0x7F80, 0x7FC0, 0x3F80)))

@@ -126,11 +126,9 @@ def test_uploaded_masks_alternate_buffers_and_match_a_direct_mask(sampler, oracl
     assert ptrs[0] == ptrs[2] and ptrs[1] == ptrs[3] and ptrs[0] != ptrs[1]
 
 
-@pytest.mark.parametrize("cap,top_k", [(32, 40), (600, 40), (32, 300)], ids=["short-ring", "long-ring", "exact-search"])
+@pytest.mark.parametrize("cap,top_k", [(32, 40), (600, 40), (32, 300)], ids=["short-ring", "long-ring", "large-top-k"])
 def test_device_history_with_one_cta_per_row(sampler, oracle, cap, top_k):
-    # 256 rows: every CTA streams one whole row (the instantiations without segment records), the
-    # CTA that finishes a row -- from its candidates or, for top-k above 256, by the exact search --
-    # appends the token to the ring; rings of at most 512 ids take the short history list
+    # 256 rows: every CTA streams one whole row and appends the token to the ring when it has finished it
     import torch
     from born_b200 import SamplingConfig, _lib as L
     B, V, steps, P = 256, 9000, 5, 20

@@ -741,8 +741,9 @@ def test_out_of_range_row_params_on_the_device_fail_their_row_only(sampler, orac
 
 
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
-def test_history_penalties_on_rows_of_more_than_64_tiles(oracle, dtype):
-    # beyond 64 tiles per row the history list is built by the hash-table path
+def test_history_penalties_on_long_rows(oracle, dtype):
+    # long rows cut into slices, each with its own part of the history list (fp32: a cluster of eight, whose
+    # values meet in the first CTA; bf16, beyond 512 blocks: records)
     from born_b200 import Sampler, SamplingConfig
     torch = torch_mod()
     B, V, H = 3, 300000 if dtype == "f32" else 600000, 700
@@ -772,9 +773,8 @@ def test_history_penalties_on_rows_of_more_than_64_tiles(oracle, dtype):
 
 @pytest.mark.parametrize("H", [512, 513, 1024])
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
-def test_history_lengths_either_side_of_the_short_list(sampler, oracle, H, dtype):
-    # 256 rows give one CTA per row; fp32 launches with at most 512 history ids per row take the
-    # instantiation with the short list and five stages, longer histories the one with four
+def test_history_lengths_with_one_cta_per_row(sampler, oracle, H, dtype):
+    # 256 rows give one CTA per row; the list's room, and with it the ring's, follows the capacity
     B, V = 256, 20000
     params = dict(temperature=0.8, min_p=0.02, top_p=0.95, repetition_penalty=1.3, frequency_penalty=0.4, presence_penalty=0.2)
     z = (W.normal(123, 1, B * V) * 3.0).astype(np.float32).reshape(B, V)
