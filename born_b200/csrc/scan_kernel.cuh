@@ -111,7 +111,7 @@ __device__ __forceinline__ int hist_shift(int span) {
 
 // The list of the distinct history tokens of blocks [j0, j1) of the row, with their multiplicities,
 // grouped by bucket.  What tells a token's first occurrence from its repeats: a bit per token of the
-// segment, where the bits fit (one atomic per id; a repeat finds its token afterwards, by a table of list
+// segment, where the bits fit and are not crowded (one atomic per id; a repeat finds its token afterwards, by a table of list
 // positions, and counts itself there), else a compare-and-swap into a hash table.  Chains of swaps
 // bound the latter, 3.6 us for 512 ids with two CTAs on an SM.  256 rows, 512 ids, hash table -> bits:
 // 32000 tokens fp32 18.9 -> 14.7 us, 128256 33.5 -> 30.4, 151936 39.5 -> 34.9; bf16 200000 45.9 -> 41.6.
@@ -121,7 +121,9 @@ __device__ __forceinline__ int hist_shift(int span) {
 __device__ __forceinline__ int hist_build(const ScanArgs& A, ScanShared& sh, uint8_t* smem, const int (&ids)[kHistPer], int g, int j0, int j1) {
     const int tid = threadIdx.x, lane = tid & 31;
     const int lg = A.L.hash_lg, slots = 1 << lg, hs = hist_shift(j1 - j0);
-    const bool bits = (j1 - j0) * (kBlkTok / 8) + kHistPos * 2 <= A.L.hash_bytes;
+    // (many ids on few words of bits queue up behind one another: 256 rows of 8192 tokens, 512 ids, take 15.1 us
+    // with the hash table and 12.5 with bits, 4096 tokens with 1024 ids 16.4 and 23.4, 1000 with 512 12.4 and 18.7)
+    const bool bits = (j1 - j0) * (kBlkTok / 8) + kHistPos * 2 <= A.L.hash_bytes && A.L.list_cap <= 64 * (j1 - j0);
     uint32_t* keys = reinterpret_cast<uint32_t*>(smem + A.L.hash);  // hash table: keys, multiplicities; or the bits
     uint32_t* mult = keys + slots;
     uint16_t* where = reinterpret_cast<uint16_t*>(keys + (j1 - j0) * (kBlkTok / 32));
